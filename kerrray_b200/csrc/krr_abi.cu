@@ -103,6 +103,10 @@ krr::Params make_params(double mass, double spin, const krr_options* o) {
   P.max_steps = o->max_steps;
   P.guard = max_attempts(o);
   P.rk4 = o->method == 1;
+  // The ranges under which the reference order's branch-free divisions neither overflow nor
+  // underflow (RefMode::metric, attempt); other scales divide by IEEE division.
+  const double big = std::ldexp(1.0, 60), small = std::ldexp(1.0, -60);
+  P.div_ok = m >= small && m <= big && (a == 0.0 || std::fabs(a) >= small) && o->atol >= std::ldexp(1.0, -400);
   P.disk = o->disk_plane != 0;
   P.r_plus = outer_horizon(m, a);
   P.f_mass = (float)m;

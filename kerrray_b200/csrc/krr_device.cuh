@@ -27,6 +27,8 @@
 #include <type_traits>
 #include <cuda_runtime.h>
 
+#include "krr_quotient.cuh"
+
 namespace krr {
 
 enum : int { RUNNING = 0, ESCAPED = 1, CAPTURED = 2, MAX_AFFINE = 3, FAILURE = 4, OUT_OF_DOMAIN = 5, DISK_HIT = 6 };
@@ -72,8 +74,9 @@ struct Params {
   double r_capture, r_escape, r_in, r_out;
   double r_plus;  // outer horizon M + sqrt(M^2 - a^2)
   long long max_steps, guard;
-  int rk4;   // 0: Dormand-Prince 5(4), 1: fixed-step RK4
-  int disk;  // disk-plane event enabled
+  short rk4;     // 0: Dormand-Prince 5(4), 1: fixed-step RK4
+  short div_ok;  // the scales allow the branch-free divisions (RefMode::metric, attempt); set by make_params
+  int disk;      // disk-plane event enabled
   // FP32 copies for the mixed mode's stages (rounded once on the host).
   float f_mass, f_a, f_a2;
   float f_rpm;  // r_plus - r_minus = 2 sqrt(M^2 - a^2)
@@ -169,25 +172,23 @@ struct RefMode {
     rhs(P, ys[CR], ys[CTH], ry.pt, ys[CPR], ys[CPTH], ry.pph, f, tr);
   }
 
-  __device__ static void metric(const Params& P, double r, double th, double g[15], Trig& tr) {
+  // The 15 metric terms' numerators and denominators in the reference's order.
+  struct Terms {
+    double sig, sd, sd2, sig2, sds2, sig2s2, sig2s4;            // denominators
+    double n0, n1, dlt, n4, n5, n6, n7, n8, n9, n10, n11, n12, n13, n14;  // numerators (n9: of a2 sd_r / sd2)
+    double m14;                                                  // numerator of a2 sd_th / sd2
+    double s2;
+  };
+  __device__ __forceinline__ static Terms terms(const Params& P, double r, double s, double c, double sin2th) {
     const double m = P.mass, a2 = P.a2;
-    const double s = sin(th);
-    const double c = cos(th);
-    tr.s = s;
-    tr.c = c;
+    Terms t;
     const double s2 = s * s;
-    const double sin2th = sin(2.0 * th);
     const double r2 = r * r;
     const double sig = r2 + a2 * (c * c);
     const double dlt = r2 - P.two_m * r + a2;
     const double r2a2 = r2 + a2;
     const double big_a = r2a2 * r2a2 - a2 * dlt * s2;
     const double sd = sig * dlt;
-    g[0] = -big_a / sd;
-    g[1] = P.neg_2ma * r / sd;
-    g[2] = dlt / sig;
-    g[3] = 1.0 / sig;
-    g[4] = (dlt - a2 * s2) / (sd * s2);
     const double sig_r = 2.0 * r;
     const double sig_th = (-a2) * sin2th;
     const double dlt_r = 2.0 * (r - m);
@@ -195,18 +196,95 @@ struct RefMode {
     const double a_th = (-a2) * dlt * sin2th;
     const double sd_r = sig_r * dlt + sig * dlt_r;
     const double sd_th = sig_th * dlt;
-    const double sd2 = sd * sd;
     const double sig2 = sig * sig;
-    g[5] = -(a_r * sd - big_a * sd_r) / sd2;
-    g[6] = P.neg_2ma * (sd - r * sd_r) / sd2;
-    g[7] = (dlt_r * sig - dlt * sig_r) / sig2;
-    g[8] = -sig_r / sig2;
-    g[9] = -sig_r / (sig2 * s2) + a2 * sd_r / sd2;
-    g[10] = -(a_th * sd - big_a * sd_th) / sd2;
-    g[11] = P.pos_2ma * r * sd_th / sd2;
-    g[12] = -dlt * sig_th / sig2;
-    g[13] = -sig_th / sig2;
-    g[14] = -(sig_th * s2 + sig * sin2th) / (sig2 * (s2 * s2)) + a2 * sd_th / sd2;
+    t.s2 = s2;
+    t.sig = sig;
+    t.sd = sd;
+    t.sd2 = sd * sd;
+    t.sig2 = sig2;
+    t.sds2 = sd * s2;
+    t.sig2s2 = sig2 * s2;
+    t.sig2s4 = sig2 * (s2 * s2);
+    t.n0 = -big_a;
+    t.n1 = P.neg_2ma * r;
+    t.dlt = dlt;
+    t.n4 = dlt - a2 * s2;
+    t.n5 = -(a_r * sd - big_a * sd_r);
+    t.n6 = P.neg_2ma * (sd - r * sd_r);
+    t.n7 = dlt_r * sig - dlt * sig_r;
+    t.n8 = -sig_r;
+    t.n9 = a2 * sd_r;
+    t.n10 = -(a_th * sd - big_a * sd_th);
+    t.n11 = P.pos_2ma * r * sd_th;
+    t.n12 = -dlt * sig_th;
+    t.n13 = -sig_th;
+    t.n14 = -(sig_th * s2 + sig * sin2th);
+    t.m14 = a2 * sd_th;
+    return t;
+  }
+
+  // Any operands, by IEEE division.  Out of line, its result by value: the operands the fast
+  // path declines are rare (a trial stage next to r = 0, the horizon or the axis, or a fraction
+  // that begins with 16 ones: one denominator in 65536).
+  struct Quotients {
+    double g[15];
+  };
+  __device__ __noinline__ static Quotients quotients_ieee(Terms t) {
+    Quotients q;
+    q.g[0] = t.n0 / t.sd;
+    q.g[1] = t.n1 / t.sd;
+    q.g[2] = t.dlt / t.sig;
+    q.g[3] = 1.0 / t.sig;
+    q.g[4] = t.n4 / t.sds2;
+    q.g[5] = t.n5 / t.sd2;
+    q.g[6] = t.n6 / t.sd2;
+    q.g[7] = t.n7 / t.sig2;
+    q.g[8] = t.n8 / t.sig2;
+    q.g[9] = t.n8 / t.sig2s2 + t.n9 / t.sd2;
+    q.g[10] = t.n10 / t.sd2;
+    q.g[11] = t.n11 / t.sd2;
+    q.g[12] = t.n12 / t.sig2;
+    q.g[13] = t.n13 / t.sig2;
+    q.g[14] = t.n14 / t.sig2s4 + t.m14 / t.sd2;
+    return q;
+  }
+
+  // The 15 terms.  The branch-free quotients hold their values while nothing overflows or
+  // underflows: with sin^2, Sigma and Sigma Delta in [2^-120, 2^120] and the mass and spin in
+  // [2^-60, 2^60] (or spin 0; P.div_ok) every denominator lies in [2^-480, 2^480], and every
+  // numerator is 0 or in [2^-700, 2^700] (products of at most six such factors; a difference that
+  // is not 0 is at least 2^-53 of its terms).
+  __device__ static void metric(const Params& P, double r, double th, double g[15], Trig& tr) {
+    const double s = sin(th);
+    const double c = cos(th);
+    tr.s = s;
+    tr.c = c;
+    const double sin2th = sin(2.0 * th);
+    const Terms t = terms(P, r, s, c, sin2th);
+    const unsigned gap = min(min(min(fraction_gap(t.sig), fraction_gap(t.sd)), min(fraction_gap(t.sd2), fraction_gap(t.sig2))),
+                             min(min(fraction_gap(t.sds2), fraction_gap(t.sig2s2)), fraction_gap(t.sig2s4)));
+    if (gap != 0u && P.div_ok && moderate(t.s2) && moderate(t.sig) && moderate(t.sd)) {
+      const Recip i_sd = recip(t.sd), i_sig = recip(t.sig), i_sd2 = recip(t.sd2), i_sig2 = recip(t.sig2);
+      g[0] = quotient(t.n0, i_sd);
+      g[1] = quotient(t.n1, i_sd);
+      g[2] = quotient(t.dlt, i_sig);
+      g[3] = quotient_one(i_sig);
+      g[4] = quotient(t.n4, t.sds2);
+      g[5] = quotient(t.n5, i_sd2);
+      g[6] = quotient(t.n6, i_sd2);
+      g[7] = quotient(t.n7, i_sig2);
+      g[8] = quotient(t.n8, i_sig2);
+      g[9] = quotient(t.n8, t.sig2s2) + quotient(t.n9, i_sd2);
+      g[10] = quotient(t.n10, i_sd2);
+      g[11] = quotient(t.n11, i_sd2);
+      g[12] = quotient(t.n12, i_sig2);
+      g[13] = quotient(t.n13, i_sig2);
+      g[14] = quotient(t.n14, t.sig2s4) + quotient(t.m14, i_sd2);
+    } else {
+      const Quotients q = quotients_ieee(t);
+#pragma unroll
+      for (int i = 0; i < 15; ++i) g[i] = q.g[i];
+    }
   }
 
   // f (6 integrated components) at state (r, th, pr, pth) with constants (pt, pph).
@@ -977,6 +1055,17 @@ __device__ __forceinline__ void dp_stages(const Params& P, const Ray<M>& ry, typ
   }
 }
 
+// The error norm's six quotients by IEEE division (out of line: scales outside the branch-free range).
+struct Six {
+  double x[NV];
+};
+static __device__ __noinline__ Six quotients_ieee(Six e, Six scale) {
+  Six v;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) v.x[i] = e.x[i] / scale.x[i];
+  return v;
+}
+
 // One step attempt (numba_kernel.py:376-455): DP5(4) (or RK4) step, error norm, controller,
 // accept/reject, diagnostics and classification.  Returns with ry.state updated.
 template <class M, bool RK4>
@@ -1016,14 +1105,42 @@ __device__ __forceinline__ void attempt(const Params& P, Ray<M>& ry, double* __r
       // modes multiply by a Newton reciprocal of the scale and compare en^2 = total / 8 with 1
       // instead of taking the square root (the step factor is a power of en^2 as well).
       N q[NV];
+      if constexpr (!M::kFused && sizeof(N) == 8) {
+        // Six independent IEEE quotients.  Branch-free (quotient) where every scale allows it: at
+        // most 2^400 here and at least atol >= 2^-400 (P.div_ok).  A numerator too small for an
+        // exact residual (below 2^-960) gives |v| < 2^-550 either way and v^2 = 0.
+        double e[NV], scale[NV];
+        unsigned gap = 0xffffffffu;
+        int top = 0;
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const K e = h * esum[i];
-        const N scale = madd<M>((N)P.atol, (N)P.rtol, py_max((N)fabs(ry.y[i]), (N)fabs(yn[i])));
-        N v;
-        if constexpr (M::kFused) v = (N)e * rcp_newton<1>(scale);
-        else v = (N)e / scale;
-        q[i] = v * v;
+        for (int i = 0; i < NV; ++i) {
+          e[i] = h * esum[i];
+          scale[i] = P.atol + P.rtol * py_max(fabs(ry.y[i]), fabs(yn[i]));
+          gap = min(gap, fraction_gap(scale[i]));
+          top = max(top, __double2hiint(scale[i]));
+        }
+        if (!(gap != 0u && top < 0x58f00000 && P.div_ok)) {  // 2^400
+          const Six v = quotients_ieee(Six{{e[0], e[1], e[2], e[3], e[4], e[5]}},
+                                       Six{{scale[0], scale[1], scale[2], scale[3], scale[4], scale[5]}});
+#pragma unroll
+          for (int i = 0; i < NV; ++i) q[i] = v.x[i] * v.x[i];
+        } else {
+#pragma unroll
+          for (int i = 0; i < NV; ++i) {
+            const double v = quotient(e[i], scale[i]);
+            q[i] = v * v;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          const K e = h * esum[i];
+          const N scale = madd<M>((N)P.atol, (N)P.rtol, py_max((N)fabs(ry.y[i]), (N)fabs(yn[i])));
+          N v;
+          if constexpr (M::kFused) v = (N)e * rcp_newton<1>(scale);
+          else v = (N)e / scale;
+          q[i] = v * v;
+        }
       }
       // Full-state slots: 0 t, 1 r, 2 th, 3 ph, 4 p_t (0), 5 p_r, 6 p_th, 7 p_phi (0).
       const N total = ((q[CT] + q[CR]) + (q[CTH] + q[CPH])) + (q[CPR] + q[CPTH]);
