@@ -1448,29 +1448,30 @@ int krr_bisect_edges(int device, const krr_edge_case* cases, int32_t n_cases, co
   if (rc) return rc;
   std::lock_guard<std::mutex> lk(ctx->mu);
   KRR_CUDA(cudaSetDevice(device));
-  // Queue order: the cases' items dealt round robin, so that every warp holds items of every
-  // tolerance, and the cheap ones, ending early, lend their lanes to the expensive ones.  That
-  // needs the cases' parameters in shared memory (krr::edge_params_in_smem); with more cases
-  // the items keep their order, and a warp's lanes mostly share a case.
-  const bool interleave = krr::edge_params_in_smem(n_cases);
+  // The items by the cost of their case, most expensive first (the DP5 step count grows like
+  // rtol^-1/5); the kernel deals them over its warps, so that every warp holds items of every
+  // tolerance and the cheap ones, ending early, lend their lanes to the expensive ones.  That
+  // needs the cases' parameters in shared memory (krr::edge_params_in_smem); with more cases the
+  // items keep their order, and a warp's lanes mostly share a case.
+  const bool deal = krr::edge_params_in_smem(n_cases);
   std::vector<long long> order((size_t)n_items);
   for (int64_t i = 0; i < n_items; ++i) order[(size_t)i] = i;
-  if (interleave) {
-    std::vector<long long> start((size_t)n_cases + 1, 0), fill((size_t)n_cases, 0);
-    for (int64_t i = 0; i < n_items; ++i) start[(size_t)item_case[i] + 1] += 1;
-    for (int k = 0; k < n_cases; ++k) start[(size_t)k + 1] += start[(size_t)k];
-    std::vector<long long> by_case((size_t)n_items);
-    for (int64_t i = 0; i < n_items; ++i) {
-      const int k = item_case[i];
-      by_case[(size_t)(start[(size_t)k] + fill[(size_t)k]++)] = i;
+  if (deal) {
+    std::vector<int> by_cost((size_t)n_cases);
+    for (int k = 0; k < n_cases; ++k) by_cost[(size_t)k] = k;
+    std::stable_sort(by_cost.begin(), by_cost.end(),
+                     [&](int x, int y) { return cases[x].options.rtol < cases[y].options.rtol; });
+    std::vector<long long> count((size_t)n_cases, 0), at((size_t)n_cases);
+    for (int64_t i = 0; i < n_items; ++i) count[(size_t)item_case[i]] += 1;
+    long long n = 0;
+    for (int k : by_cost) {
+      at[(size_t)k] = n;
+      n += count[(size_t)k];
     }
-    size_t n = 0;
-    for (long long r = 0; n < (size_t)n_items; ++r)
-      for (int k = 0; k < n_cases; ++k)
-        if (start[(size_t)k] + r < start[(size_t)k + 1]) order[n++] = by_case[(size_t)(start[(size_t)k] + r)];
+    for (int64_t i = 0; i < n_items; ++i) order[(size_t)at[(size_t)item_case[i]]++] = i;
   }
   const size_t nb8 = (size_t)n_items * 8, nb4 = (size_t)n_items * 4;
-  const size_t bytes = 512 + round256((size_t)n_cases * sizeof(krr::EdgeCase)) + 6 * round256(nb8) + round256(nb4);
+  const size_t bytes = 512 + round256((size_t)n_cases * sizeof(krr::EdgeCase)) + 7 * round256(nb8) + round256(nb4);
   KRR_CUDA(ctx->buf[B_AB].ensure(bytes));
   char* base = static_cast<char*>(ctx->buf[B_AB].p);
   krr::Queue* d_q = reinterpret_cast<krr::Queue*>(base);
@@ -1484,6 +1485,7 @@ int krr_bisect_edges(int device, const krr_edge_case* cases, int32_t n_cases, co
   auto* d_hi = reinterpret_cast<double*>(take(nb8));
   auto* d_fail = reinterpret_cast<long long*>(take(nb8));
   auto* d_order = reinterpret_cast<long long*>(take(nb8));
+  auto* d_star = reinterpret_cast<double*>(take(nb8));
   const cudaStream_t s = ctx->stream;
   KRR_CUDA(cudaMemsetAsync(d_q, 0, sizeof(krr::Queue), s));
   KRR_CUDA(cudaMemcpyAsync(d_cases, ec.data(), ec.size() * sizeof(krr::EdgeCase), cudaMemcpyHostToDevice, s));
@@ -1502,12 +1504,15 @@ int krr_bisect_edges(int device, const krr_edge_case* cases, int32_t n_cases, co
   a.hi = d_hi;
   a.failures = d_fail;
   a.order = d_order;
+  a.deal = deal;
+  a.star = d_star;
   a.n_cases = n_cases;
   a.n_items = n_items;
   a.iterations = iterations;
   a.q = d_q;
   a.refill_threshold = 1;
   KRR_CUDA(cudaEventRecord(ctx->ev0, s));
+  KRR_CUDA(krr::edge_predict(a, s));
   KRR_CUDA(precision == KRR_PREC_REFERENCE ? krr::ref_bisect(a, s) : krr::fast_bisect(precision == KRR_PREC_MIXED, a, s));
   KRR_CUDA(cudaEventRecord(ctx->ev1, s));
   krr::Queue q{};

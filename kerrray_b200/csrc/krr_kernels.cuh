@@ -286,20 +286,31 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // traced; ESCAPED moves hi to mid, anything else moves lo to mid; a result that is neither
 // ESCAPED nor CAPTURED counts as a failure.
 //
-// One lane owns an item and runs its halvings one after another.  Once the queue is drained,
-// a warp's idle lanes trace ahead: a helper takes a node of the bisection tree below an
-// owner's current bracket, at depth 1..KRR_EDGE_DEPTH (the brackets the item holds after the
-// owner's photon and the next ones, for either outcome), and traces its midpoint while the
-// owner's photon is still running.  When the owner's photon ends, the helpers on the outcome's
-// side move up one level; the one at depth 1 inherits the item and continues with its photon
-// (possibly already ended, which settles one more halving at once); the helpers on the other
-// side are discarded.  Every midpoint is 0.5 * (lo + hi) of the bracket the sequential
-// bisection would hold there, so the results are the sequential ones bit for bit.  Lanes are
-// given to the shallowest untraced nodes first, across the warp's owners with the most work
-// left, then across the others.  A warp's lanes share its instructions, so a helper costs
-// issue slots only where its warp would otherwise have ended; the host interleaves the items
-// of all cases so that every warp holds cheap items, which end early and lend their lanes,
-// beside expensive ones.
+// One lane owns an item and runs its halvings one after another.  A warp takes at most
+// ceil(items / warps) items, so that a study smaller than the grid is spread over every warp, and
+// its other lanes trace ahead: a helper takes a node of the bisection tree below an owner's
+// current bracket, at some depth d (the bracket the item holds after the owner's photon and the
+// next d - 1 ones), and traces its midpoint while the owner's photon is still running.  When the
+// owner's photon ends, the helpers on the outcome's side move up one level; the one at depth 1
+// inherits the item and continues with its photon (possibly already ended, which settles one more
+// halving at once); the helpers on the other side are discarded.  Every midpoint is
+// 0.5 * (lo + hi) of the bracket the sequential bisection would hold there, so the results are the
+// sequential ones bit for bit.
+//
+// Which nodes are worth tracing is predicted: k_edge_predict finds each item's analytic edge
+// radius `star` from the constants of motion, and a photon further than EDGE_CONF * rtol M from
+// it almost surely ends on its analytic side (the integration moves the edge by about 2 rtol M; a
+// bracket that no longer holds `star` widens the doubt).  The nodes along the predicted path, down
+// to the first photon closer than that (its length is the owner's `chain`: about 20 levels of a
+// 6 M bracket at rtol 1e-6, 31 at 1e-10), are traced first, then the tree below the path's end,
+// where either outcome is possible.  A wrong prediction costs the attempts of the nodes below it,
+// nothing else.
+//
+// Measured (kernel, B200).  One edge, 90 directions, 36 halvings, rtol 1e-6, reference order: 87 ms
+// with the first three warps holding every item, 20 ms now (2000 attempts per warp for 36 halvings
+// of 341 each).  12 cases x 241 directions x 3 tolerances, fast64: 110 -> 36 ms; with the items in
+// runs of one tolerance instead of dealt, 52 ms.  x 1440 directions (51,840 items, every lane an
+// owner until the queue is drained): 127 -> 116 ms.  EDGE_CONF 2 and 16 within 5 % of 4 on all three.
 // ------------------------------------------------------------------------------------------
 struct EdgeCase {
   Params P;
@@ -315,7 +326,9 @@ struct EdgeArgs {
   double* lo;
   double* hi;
   long long* failures;
-  const long long* order;  // queue position -> item (nullable: identity)
+  const long long* order;  // the items, most expensive first
+  bool deal;               // deal them over the warps (otherwise in order)
+  double* star;            // predicted edge radius of each item (k_edge_predict)
   int n_cases;
   long long n_items;
   int iterations;
@@ -327,7 +340,7 @@ struct EdgeArgs {
 template <class M>
 struct EdgeLane {
   Ray<M> ry;
-  double lo, hi, mid, cphi, sphi;
+  double lo, hi, mid, cphi, sphi, star;
   long long fails;
   int it, c;
 };
@@ -345,14 +358,14 @@ __device__ __forceinline__ void edge_start(const EdgeArgs& a, EdgeLane<M>& L) {
 
 enum : int { EDGE_IDLE = 0, EDGE_OWNER = 1, EDGE_HELPER = 2 };
 
-#ifndef KRR_EDGE_DEPTH
-#define KRR_EDGE_DEPTH 4
-#endif
-// Nodes below an owner's bracket, depth d = 1..KRR_EDGE_DEPTH, path p (d bits, the first step
-// in the highest bit; 1 = the photon before escaped): bit (2^d - 2 + p) of a 32-bit mask.
-constexpr int EDGE_DEPTH = KRR_EDGE_DEPTH;
-static_assert(EDGE_DEPTH >= 1 && EDGE_DEPTH <= 4, "the node masks hold depths 1..4");
-__device__ __forceinline__ int edge_node(int d, int p) { return (1 << d) - 2 + p; }
+// A node below an owner's bracket: depth d >= 1 and path p, d bits, the first step in the highest
+// (1 = the photon before escaped); d <= EDGE_CHAIN.  The tree below the predicted path's end is
+// traced EDGE_DEPTH levels deep, its node t levels below the end with path bits p being bit
+// (2^t - 2 + p) of a 32-bit mask.
+constexpr int EDGE_DEPTH = 4, EDGE_CHAIN = 31;
+constexpr double EDGE_CONF = 4.0;  // of rtol M: nearer to the predicted edge, either outcome is possible
+constexpr double EDGE_OFF = 3.0;   // of the least error of the prediction that the bracket shows
+__device__ __forceinline__ int edge_node(int d, unsigned p) { return (1 << d) - 2 + (int)p; }
 
 __device__ __forceinline__ int nth_set_bit(unsigned mask, int n) {
   for (int i = 0; i < n; ++i) mask &= mask - 1u;
@@ -385,16 +398,30 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
     if constexpr (SMEM) return s_params[c];
     else return a.cases[c].P;
   };
-  __shared__ int slots[MAXT];  // 32 per warp, indexed by lane
-  int* slot = slots + (threadIdx.x & ~31u);
+  __shared__ int slots[2 * MAXT];  // 64 per warp, two indexed by lane
+  int* slot = slots + 2 * (threadIdx.x & ~31u);
+  int* slot2 = slot + 32;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
   EdgeLane<M> L;
   L.ry.state = FAILURE;
-  L.lo = L.hi = L.mid = L.cphi = L.sphi = 0.0;
+  L.lo = L.hi = L.mid = L.cphi = L.sphi = L.star = 0.0;
   L.fails = 0;
   L.it = L.c = 0;
-  int role = EDGE_IDLE, host = 0, depth = 0, path = 0;
+  int role = EDGE_IDLE, host = 0, depth = 0;
+  unsigned path = 0;
+  const long long warps = (long long)gridDim.x * (MAXT / 32);
+  const int cap = (int)min(32LL, (a.n_items + warps - 1) / warps);  // items a warp holds at a time
+  // The queue deals the items, ordered by cost, like cards: a run of cap queue positions (a warp's
+  // first items) takes every `columns`-th item, so that each warp holds items of every cost.
+  const long long columns = a.deal ? (a.n_items + cap - 1) / cap : a.n_items, rows = a.n_items / columns,
+                  longer = a.n_items % columns;  // the first `longer` columns hold one item more
+  auto dealt = [&](long long pos) {
+    const long long head = longer * (rows + 1);
+    const long long w = pos < head ? pos / (rows + 1) : longer + (pos - head) / rows;
+    const long long j = pos < head ? pos % (rows + 1) : (pos - head) % rows;
+    return j * columns + w;
+  };
   bool drained = false, dirty = true;
   long long g = -1;
   unsigned long long my_attempts = 0, my_accepted = 0, my_spec = 0, my_discarded = 0;
@@ -428,7 +455,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
       const int hl = (role == EDGE_HELPER) ? host : (int)lane;
       const int host_want = __shfl_sync(FULL, want, hl);
       const bool host_ended = role == EDGE_HELPER && ((em >> hl) & 1u);
-      const bool on_side = host_ended && host_want >= 0 && ((path >> (depth - 1)) & 1) == host_want;
+      const bool on_side = host_ended && host_want >= 0 && (int)((path >> (depth - 1)) & 1u) == host_want;
       const bool heir = on_side && depth == 1;
       if (heir) slot[host] = (int)lane;
       __syncwarp();
@@ -437,19 +464,21 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
       const int src = heir ? host : (int)lane;
       const double lo_s = __shfl_sync(FULL, L.lo, src);
       const double hi_s = __shfl_sync(FULL, L.hi, src);
+      const double star_s = __shfl_sync(FULL, L.star, src);
       const long long fails_s = __shfl_sync(FULL, L.fails, src);
       const long long g_s = __shfl_sync(FULL, g, src);
       const int it_s = __shfl_sync(FULL, L.it, src);
       if (heir) {  // the item's bracket is this lane's: its midpoint is this photon's
         L.lo = lo_s;
         L.hi = hi_s;
+        L.star = star_s;
         L.fails = fails_s;
         L.it = it_s;
         g = g_s;
         role = EDGE_OWNER;
       } else if (on_side) {  // one level up, below the heir (or the same owner)
         depth -= 1;
-        path &= (1 << depth) - 1;
+        path &= (1u << depth) - 1u;
         if (new_host >= 0) host = new_host;
       } else if (host_ended) {  // the other side: the photon is not needed
         my_discarded += (unsigned long long)L.ry.attempts;
@@ -468,22 +497,25 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
     // New items from the queue for idle lanes.
     const unsigned idle = __ballot_sync(FULL, role == EDGE_IDLE);
     const int n_idle = __popc(idle);
-    if (!drained && n_idle > 0 && (n_idle >= a.refill_threshold || n_idle == 32)) {
+    const int want_items = min(n_idle, cap - __popc(__ballot_sync(FULL, role == EDGE_OWNER)));
+    if (!drained && want_items > 0 && (n_idle >= a.refill_threshold || n_idle == 32)) {
       dirty = true;
       unsigned long long base = 0;
       const int leader = __ffs(idle) - 1;
-      if ((int)lane == leader) base = atomicAdd(&a.q->head, (unsigned long long)n_idle);
+      if ((int)lane == leader) base = atomicAdd(&a.q->head, (unsigned long long)want_items);
       base = __shfl_sync(FULL, base, leader);
-      if (base + (unsigned long long)n_idle >= (unsigned long long)a.n_items) drained = true;
-      if (role == EDGE_IDLE) {
-        const unsigned long long mine = base + (unsigned long long)__popc(idle & lt_mask);
+      if (base + (unsigned long long)want_items >= (unsigned long long)a.n_items) drained = true;
+      const int rank = __popc(idle & lt_mask);
+      if (role == EDGE_IDLE && rank < want_items) {
+        const unsigned long long mine = base + (unsigned long long)rank;
         if (mine < (unsigned long long)a.n_items) {
-          g = a.order ? a.order[mine] : (long long)mine;
+          g = a.order[dealt((long long)mine)];
           L.c = a.item_case[g];
           L.lo = a.lo[g];
           L.hi = a.hi[g];
           L.cphi = a.cos_phi[g];
           L.sphi = a.sin_phi[g];
+          L.star = a.star[g];
           L.fails = 0;
           L.it = 0;
           role = EDGE_OWNER;
@@ -493,21 +525,65 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
       }
       resolve();
     }
-    // Once the queue is drained: idle lanes take the untraced nodes below the owners'
-    // brackets, shallowest first, then in lane order of the owners.
-    if (drained && dirty) {
+    // With no more items to take: idle lanes take the untraced nodes below the owners' brackets,
+    // along the predicted paths first, shallowest first, then in lane order of the owners.
+    if (dirty && (drained || __popc(__ballot_sync(FULL, role == EDGE_OWNER)) >= cap)) {
       dirty = false;
       const unsigned idle2 = __ballot_sync(FULL, role == EDGE_IDLE);
+      const int n_idle2 = __popc(idle2);
       if (idle2) {
-        slot[lane] = 0;
+        // The owners' predicted paths.
+        int chain = 0;
+        unsigned cpath = 0;
+        const int below = (role == EDGE_OWNER) ? a.iterations - 1 - L.it : 0;  // levels below the owner's photon
+        if (below > 0) {
+          const Params& Pc = params(L.c);
+          // a bracket that no longer holds `star` shows how far off it is at least
+          const double off = fmax(fmax(L.lo - L.star, L.star - L.hi), 0.0);
+          const double conf = EDGE_CONF * Pc.rtol * Pc.mass + EDGE_OFF * off;
+          const int most = min(below, EDGE_CHAIN);
+          double lo_c = L.lo, hi_c = L.hi, mid = L.mid;
+          while (chain < most && fabs(mid - L.star) > conf) {
+            const bool out = mid > L.star;
+            cpath = 2u * cpath + (out ? 1u : 0u);
+            if (out) hi_c = mid; else lo_c = mid;
+            chain += 1;
+            mid = 0.5 * (lo_c + hi_c);
+          }
+        }
+        slot[lane] = slot2[lane] = 0;
         __syncwarp();
-        if (role == EDGE_HELPER) atomicOr(&slot[host], 1 << edge_node(depth, path));
+        {
+          const int src = (role == EDGE_HELPER) ? host : (int)lane;
+          const int ch = __shfl_sync(FULL, chain, src);
+          const unsigned cp = __shfl_sync(FULL, cpath, src);
+          if (role == EDGE_HELPER) {
+            if (depth <= ch) {
+              if (path == cp >> (ch - depth)) atomicOr(&slot[host], (int)(1u << (depth - 1)));
+            } else if (depth - ch <= EDGE_DEPTH && path >> (depth - ch) == cp) {
+              atomicOr(&slot2[host], 1 << edge_node(depth - ch, path & ((1u << (depth - ch)) - 1u)));
+            }
+          }
+        }
         __syncwarp();
-        const unsigned cover = (unsigned)slot[lane];
+        const unsigned on_chain = (unsigned)slot[lane], in_tree = (unsigned)slot2[lane];
         const int rank = (role == EDGE_IDLE) ? __popc(idle2 & lt_mask) : -1;
-        // The owners with the most work left (halvings left x rtol^-1/5, the DP5 step count's
-        // growth) come first: those at least half the warp's largest, then the others (5 % of
-        // the edge study's time, 17 % fewer attempts discarded).
+        int h = -1, hd = 0, base_rank = 0;  // the node taken: owner lane, depth, path
+        unsigned hp = 0;
+        const int longest = __reduce_max_sync(FULL, chain);
+        for (int d = 1; d <= longest && base_rank < n_idle2; ++d) {
+          const unsigned open = __ballot_sync(FULL, d <= chain && !((on_chain >> (d - 1)) & 1u));
+          const int key = rank - base_rank;
+          if (h < 0 && key >= 0 && key < __popc(open)) {
+            h = nth_set_bit(open, key);
+            hd = d;
+          }
+          base_rank += __popc(open);
+        }
+        // The tree below the paths' ends.  The owners with the most work left (halvings left x
+        // rtol^-1/5, the DP5 step count's growth) come first: those at least half the warp's
+        // largest, then the others.
+        const bool in_chain = h >= 0;
         float work = 0.0f;
         if (role == EDGE_OWNER)
           work = (float)(a.iterations - L.it) * exp2f(-0.2f * __log2f((float)params(L.c).rtol));
@@ -515,21 +591,19 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(FULL, wmax, off));
         const bool heavy = work >= 0.5f * wmax;
-        int h = -1, hd = 0, hp = 0, base_rank = 0;
-#pragma unroll
-        for (int pd = 0; pd < 2 * EDGE_DEPTH; ++pd) {
-          const int d = pd % EDGE_DEPTH + 1;
+        for (int pd = 0; pd < 2 * EDGE_DEPTH && base_rank < n_idle2; ++pd) {
+          const int t = pd % EDGE_DEPTH + 1;
           const bool this_pass = (pd < EDGE_DEPTH) == heavy;
-          const int width = 1 << d;
+          const int width = 1 << t;
           unsigned seg = 0;
-          if (role == EDGE_OWNER && this_pass && L.it + d < a.iterations)
-            seg = (~cover >> (width - 2)) & (width == 32 ? FULL : ((1u << width) - 1u));
+          if (role == EDGE_OWNER && this_pass && chain + t <= min(below, EDGE_CHAIN))
+            seg = (~in_tree >> (width - 2)) & ((1u << width) - 1u);
           const int cnt = __popc(seg);
           int incl = cnt;
 #pragma unroll
           for (int off = 1; off < 32; off <<= 1) {
-            const int t = __shfl_up_sync(FULL, incl, off);
-            if ((int)lane >= off) incl += t;
+            const int u = __shfl_up_sync(FULL, incl, off);
+            if ((int)lane >= off) incl += u;
           }
           const int total = __shfl_sync(FULL, incl, 31);
           const bool mine = h < 0 && rank >= base_rank && rank < base_rank + total;
@@ -544,8 +618,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
           const unsigned seg_j = __shfl_sync(FULL, seg, j);
           if (mine) {
             h = j;
-            hd = d;
-            hp = nth_set_bit(seg_j, key - excl_j);
+            hd = t;
+            hp = (unsigned)nth_set_bit(seg_j, key - excl_j);
           }
           base_rank += total;
         }
@@ -556,11 +630,19 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
         const double sphi_s = __shfl_sync(FULL, L.sphi, src);
         const int c_s = __shfl_sync(FULL, L.c, src);
         const int it_s = __shfl_sync(FULL, L.it, src);
+        const int ch_s = __shfl_sync(FULL, chain, src);
+        const unsigned cp_s = __shfl_sync(FULL, cpath, src);
         if (h >= 0) {
+          if (in_chain) {
+            hp = cp_s >> (ch_s - hd);
+          } else {
+            hp |= cp_s << hd;
+            hd += ch_s;
+          }
           // the brackets along the path from the owner's: escaped halves to [lo, mid]
           for (int k = hd - 1; k >= 0; --k) {
             const double mid = 0.5 * (lo_s + hi_s);
-            if ((hp >> k) & 1) hi_s = mid; else lo_s = mid;
+            if ((hp >> k) & 1u) hi_s = mid; else lo_s = mid;
           }
           L.lo = lo_s;
           L.hi = hi_s;
@@ -640,6 +722,11 @@ cudaError_t run_bisect(EdgeArgs a, cudaStream_t s) {
   return edge_params_in_smem(a.n_cases) ? run_bisect_as<M, MAXT, MINB, true>(a, s)
                                         : run_bisect_as<M, MAXT, MINB, false>(a, s);
 }
+
+// The analytic edge radius of every item into a.star (see k_bisect_edges): NaN where the ends'
+// analytic classes are not "captured at lo, escaped at hi", +-infinity where both are the same.
+__global__ void k_edge_predict(EdgeArgs a);
+cudaError_t edge_predict(const EdgeArgs& a, cudaStream_t s);
 
 // Flag the pixels whose classification the FP64 re-trace must settle: every photon that did not
 // end ESCAPED or CAPTURED, and every pixel with a different code from one of its 8 neighbours

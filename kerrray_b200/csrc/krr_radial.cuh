@@ -77,18 +77,15 @@ KRR_HD inline int radial_minima(const RadialPoly& R, double out[2]) {
   return n;
 }
 
-// RISK_ESCAPE / RISK_CAPTURE for a photon whose analytic class holds with a margin of tau_b
-// (M) in the image plane, RISK_CRITICAL otherwise.  Only photons moving inward (p_r < 0) from
-// outside the capture radius, with |L| not negligible against their impact parameter (an
-// axis-crossing ray ends OUT_OF_DOMAIN), are classified; anything else, and any non-finite
-// intermediate, is critical.
-// With tau_near > tau_b, an escaping photon within tau_near of the boundary is RISK_NEAR.
-KRR_HD inline int radial_risk(double mass, double a, double r_capture, const double y0[8], double tau_b,
-                              double tau_near = 0.0) {
+// The radial potential's minimum over [r_capture, r0] (negative: the photon turns around and
+// escapes) and its sensitivity to the image point: |vmin| / sens is the first-order distance to
+// the boundary.  False for a photon that is not classified (radial_risk).
+KRR_HD inline bool radial_margin(double mass, double a, double r_capture, const double y0[8], double* vmin_out,
+                                 double* sens_out) {
   const double r0 = y0[1], th = y0[2], pt = y0[4], pr = y0[5], pth = y0[6], pph = y0[7];
-  if (!(pr < 0.0) || !(r0 > r_capture)) return RISK_CRITICAL;
+  if (!(pr < 0.0) || !(r0 > r_capture)) return false;
   const double e = -pt;
-  if (!(e != 0.0)) return RISK_CRITICAL;
+  if (!(e != 0.0)) return false;
   const double s = sin(th), c = cos(th);
   const double lz2_over_s2 = (pph != 0.0) ? (pph * pph) / (s * s) : 0.0;
   const double q = pth * pth + (c * c) * (lz2_over_s2 - a * a * e * e);
@@ -96,7 +93,7 @@ KRR_HD inline int radial_risk(double mass, double a, double r_capture, const dou
   const double eta = q / (e * e);
   const double a2 = a * a;
   const double b = sqrt(fmax(eta + lam * lam, 0.0));
-  if (!(fabs(lam) > 1e-6 * b)) return RISK_CRITICAL;
+  if (!(fabs(lam) > 1e-6 * b)) return false;
   RadialPoly R;
   R.c2 = a2 - lam * lam - eta;
   R.c1 = 2.0 * mass * (eta + (lam - a) * (lam - a));
@@ -117,7 +114,21 @@ KRR_HD inline int radial_risk(double mass, double a, double r_capture, const dou
   const double dlt = fma(rm, rm - 2.0 * mass, a2);
   const double dr_deta = -dlt;
   const double dr_dlam = -2.0 * a * (rm * rm + a2 - a * lam) - 2.0 * dlt * (lam - a);
-  const double sens = fabs(dr_dlam) + 2.0 * b * fabs(dr_deta);
+  *vmin_out = vmin;
+  *sens_out = fabs(dr_dlam) + 2.0 * b * fabs(dr_deta);
+  return true;
+}
+
+// RISK_ESCAPE / RISK_CAPTURE for a photon whose analytic class holds with a margin of tau_b
+// (M) in the image plane, RISK_CRITICAL otherwise.  Only photons moving inward (p_r < 0) from
+// outside the capture radius, with |L| not negligible against their impact parameter (an
+// axis-crossing ray ends OUT_OF_DOMAIN), are classified; anything else, and any non-finite
+// intermediate, is critical.
+// With tau_near > tau_b, an escaping photon within tau_near of the boundary is RISK_NEAR.
+KRR_HD inline int radial_risk(double mass, double a, double r_capture, const double y0[8], double tau_b,
+                              double tau_near = 0.0) {
+  double vmin, sens;
+  if (!radial_margin(mass, a, r_capture, y0, &vmin, &sens)) return RISK_CRITICAL;
   if (!(fabs(vmin) > tau_b * sens)) return RISK_CRITICAL;
   if (vmin < 0.0 && !(fabs(vmin) > tau_near * sens)) return RISK_NEAR;
   return vmin < 0.0 ? RISK_ESCAPE : RISK_CAPTURE;

@@ -1,6 +1,8 @@
 // Kernels in the reference's operation order.  This translation unit is compiled with
 // -fmad=false: every product and sum is rounded separately, as in KerrRay's Numba kernel
 // (fastmath=False, src/kerrray/raytracing/backends/numba_kernel.py:466).
+#include <math_constants.h>
+
 #include "krr_launch.h"
 
 namespace krr {
@@ -27,6 +29,56 @@ cudaError_t ref_bisect(const EdgeArgs& a, cudaStream_t s) { return run_bisect<Re
 const Variant* ref_wide_variant() {
   static const Variant v = make_variant<RefMode<double>, false, 256, 1>();
   return &v;
+}
+
+// One item per thread: where the radial potential's minimum changes sign between the ends of the
+// bracket, by 8 halvings and 6 regula falsi steps (Illinois: an end kept twice counts half), which
+// reach about 1e-13 M.  About 30 us whatever the study's size (one chain of 16 evaluations).
+__global__ void __launch_bounds__(128) k_edge_predict(EdgeArgs a) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= a.n_items) return;
+  const EdgeCase& ec = a.cases[a.item_case[i]];
+  const double cphi = a.cos_phi[i], sphi = a.sin_phi[i];
+  auto margin = [&](double rho) {  // > 0 captured, < 0 escapes, NaN not classified
+    double y0[8], vmin, sens;
+    camera_state(ec.F, ec.c_alpha + rho * cphi, ec.c_beta + rho * sphi, y0);
+    if (!radial_margin(ec.P.mass, ec.P.a, ec.P.r_capture, y0, &vmin, &sens)) return CUDART_NAN;
+    return vmin / sens;
+  };
+  double lo = a.lo[i], hi = a.hi[i];
+  double f_lo = margin(lo), f_hi = margin(hi);
+  double star = CUDART_NAN;
+  if (f_lo < 0.0 && f_hi < 0.0) {
+    star = -CUDART_INF;
+  } else if (f_lo >= 0.0 && f_hi >= 0.0) {
+    star = CUDART_INF;
+  } else if (f_lo >= 0.0 && f_hi < 0.0) {
+    int kept = 0;  // the end the last regula falsi step left: -1 hi, +1 lo
+    for (int k = 0; k < 14; ++k) {
+      const double x = k < 8 ? 0.5 * (lo + hi) : lo + (hi - lo) * (f_lo / (f_lo - f_hi));
+      const double f = margin(x);
+      star = x;
+      if (f < 0.0) {
+        hi = x;
+        f_hi = f;
+        if (k >= 8 && kept == 1) f_lo *= 0.5;
+        kept = k >= 8 ? 1 : 0;
+      } else {
+        lo = x;
+        f_lo = f;
+        if (k >= 8 && kept == -1) f_hi *= 0.5;
+        kept = k >= 8 ? -1 : 0;
+      }
+    }
+  }
+  a.star[i] = star;
+}
+
+cudaError_t edge_predict(const EdgeArgs& a, cudaStream_t s) {
+  if (a.n_items <= 0) return cudaSuccess;
+  const int block = 128;
+  k_edge_predict<<<(unsigned)((a.n_items + block - 1) / block), block, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 // Warp-aggregated append of the flagged lanes' global indices to list (count in q->flagged).
