@@ -139,8 +139,10 @@ typedef struct krr_image {
 typedef struct krr_launch {
   int32_t precision;         /* KRR_PREC_* */
   int32_t block;             /* threads per block */
-  int32_t blocks_per_sm;     /* resident blocks per SM */
-  int32_t refill_threshold;  /* idle lanes of a warp before it refills from the queue */
+  int32_t blocks_per_sm;     /* resident blocks per SM (0: as many as fit) */
+  int32_t refill_threshold;  /* idle lanes of a warp before it refills from the queue (0: 1); with
+                                blocks_per_sm, refill_threshold and variant all 0 the library
+                                chooses the three for the number of photons */
   int32_t plain;             /* 1: one thread per photon, no work queue (the plain kernel) */
   int32_t variant;           /* compiled launch shape of the persistent kernel (krr_list_variants) */
   int32_t retrace;           /* KRR_RETRACE_*: settle the pixels a mixed trace could classify

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <thread>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -443,29 +444,55 @@ int build_images(const krr_image* images, int32_t n_images, std::vector<krr::Ima
   return KRR_OK;
 }
 
-struct LaunchShape {
-  const krr::Variant* v;
-  int grid, refill;
-};
-
 const krr::Variant* variants_for(int32_t precision, const krr_options* o, int* count) {
   const bool rk4 = o->method == 1;
   if (precision == KRR_PREC_REFERENCE) return krr::ref_variants(o->dtype == 1, rk4, count);
   return krr::fast_variants(precision == KRR_PREC_MIXED, rk4, count);
 }
 
-int persistent_shape(int device, int32_t precision, const krr_options* o, const krr_launch* l, LaunchShape& s) {
+// The launch shape a caller asked for or, with none of variant, blocks_per_sm and refill_threshold
+// set, the library's for `total` photons (each measured on the B200; the results never differ):
+// - a queue that fits the lanes of the shape without a register cap (variant 0: fast64 2 blocks of
+//   128 per SM, mixed 3, reference 2) is bound by its longest photon's chain of steps, and that
+//   shape has the shortest: 100^2 photons in fast64 0.69 ms against 0.78-0.83 at 12 warps per SM.
+//   It gets only the blocks it fills, so that no scheduler holds two warps while others idle:
+//   0.69 -> 0.57 ms, reference order 2.42 -> 2.06.
+// - a longer queue is bound by throughput: variant 1 (fast64 168 registers, 12 warps per SM; mixed
+//   128, 16 warps), and idle lanes wait until several can be refilled together, since a photon's
+//   start costs its warp about as much as a step attempt (the reference order's more than one).
+//   12.4M photons in fast64 221 ms (variant 0, refilling at 1 idle lane), 188 (variant 1), 166.5
+//   (at 6); 172.9 at 2, 171.2 at 8. Mixed 1024^2 7.34 -> 5.91 ms. At 300^2 (90k photons, 2.4 per
+//   lane of variant 0) fast64 1.22 -> 1.07 ms, mixed the same either way. Reference order 600^2:
+//   21.4 ms at 1, 16.0 at 4, 14.3 at 8, 13.8 at 12 (300^2: 5.2, 4.8, 4.6, 4.6).
+int persistent_shape(int device, int32_t precision, const krr_options* o, const krr_launch* l, long long total,
+                     LaunchShape& s) {
   int count = 0;
   const krr::Variant* vs = variants_for(precision, o, &count);
   if (!vs || count < 1) return fail(KRR_ERR_UNSUPPORTED, "no persistent kernel for this precision/method");
-  const int idx = (l && l->variant > 0) ? l->variant : 0;
+  int idx = (l && l->variant > 0) ? l->variant : 0;
   if (idx >= count) return fail(KRR_ERR_INVALID, "launch variant %d out of range [0, %d)", idx, count);
+  const bool chosen = l && (l->variant > 0 || l->blocks_per_sm > 0 || l->refill_threshold > 0);
+  const long long sms = sm_count_of(device);
+  int occ = vs[idx].occupancy();
+  bool fits = true;
+  if (!chosen) {
+    fits = total <= sms * std::max(occ, 0) * vs[0].block;
+    if (!fits && count > 1) {
+      idx = 1;
+      occ = vs[idx].occupancy();
+    }
+  }
   s.v = &vs[idx];
-  int occ = s.v->occupancy();
   if (occ < 1) return fail(KRR_ERR_CUDA, "persistent kernel variant %d cannot be resident on this device", idx);
-  const int bps = (l && l->blocks_per_sm > 0) ? std::min(l->blocks_per_sm, occ) : occ;
-  s.grid = sm_count_of(device) * bps;
-  s.refill = (l && l->refill_threshold > 0) ? std::min(l->refill_threshold, 32) : 1;
+  if (chosen) {
+    const int bps = l->blocks_per_sm > 0 ? std::min(l->blocks_per_sm, occ) : occ;
+    s.grid = (int)sms * bps;
+    s.refill = l->refill_threshold > 0 ? std::min(l->refill_threshold, 32) : 1;
+  } else {
+    const long long per_layer = sms * s.v->block;
+    s.grid = (int)(sms * (fits ? std::min<long long>(occ, std::max(1LL, (total + per_layer - 1) / per_layer)) : occ));
+    s.refill = fits ? 1 : (precision == KRR_PREC_REFERENCE ? 8 : 6);
+  }
   return KRR_OK;
 }
 
@@ -586,7 +613,7 @@ int prepare_pipeline(int device, const krr_image* images, int n_images, long lon
   p.w = work_layout(d_work, n_images, p.retrace ? total : 0);
   p.out = *d_out;
   LaunchShape shape{};
-  rc = persistent_shape(device, precision, o0, launch, shape);
+  rc = persistent_shape(device, precision, o0, launch, total, shape);
   if (rc) return rc;
   p.main_v = shape.v;
   p.main.images = p.w.images;
@@ -600,9 +627,7 @@ int prepare_pipeline(int device, const krr_image* images, int n_images, long lon
   p.main.block = shape.v->block;
   if (p.retrace) {
     LaunchShape rs{};
-    krr_launch rl{};
-    rl.precision = KRR_PREC_REFERENCE;
-    rc = persistent_shape(device, KRR_PREC_REFERENCE, o0, &rl, rs);
+    rc = persistent_shape(device, KRR_PREC_REFERENCE, o0, nullptr, LLONG_MAX, rs);  // every resident block
     if (rc) return rc;
     p.re_v = rs.v;
     p.re = p.main;

@@ -88,11 +88,10 @@ extern "C" int krr_trace_images_noalloc(int device, const krr_image* images, int
   }
   int rc = check_precision(precision, &images[0].options);
   if (rc) return rc;
-  int count = 0;
-  const krr::Variant* vs = variants_for(precision, &images[0].options, &count);
-  const int idx = (launch && launch->variant > 0) ? launch->variant : 0;
-  if (!vs || idx >= count) return fail(KRR_ERR_INVALID, "launch variant %d out of range [0, %d)", idx, count);
   if (cudaSetDevice(device) != cudaSuccess) return fail(KRR_ERR_NO_DEVICE, "cannot select device %d", device);
+  LaunchShape shape{};
+  rc = persistent_shape(device, precision, &images[0].options, launch, total, shape);
+  if (rc) return rc;
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
@@ -110,8 +109,6 @@ extern "C" int krr_trace_images_noalloc(int device, const krr_image* images, int
   if (e == cudaSuccess && d_out->event_Y) e = cudaMemsetAsync(d_out->event_Y, 0, (size_t)total * 8 * sizeof(double), s);
   if (e == cudaSuccess && d_out->event_hit) e = cudaMemsetAsync(d_out->event_hit, 0, (size_t)total, s);
   if (e != cudaSuccess) return fail(KRR_ERR_CUDA, "scratch upload: %s", cudaGetErrorString(e));
-  const int occ = vs[idx].occupancy();
-  if (occ < 1) return fail(KRR_ERR_CUDA, "persistent kernel variant %d cannot be resident", idx);
   krr::PersistArgs a{};
   a.images = d_images;
   a.n_images = n_images;
@@ -119,10 +116,10 @@ extern "C" int krr_trace_images_noalloc(int device, const krr_image* images, int
   a.Y0 = d_Y0;
   a.o = to_outputs(d_out);
   a.q = d_q;
-  a.refill_threshold = (launch && launch->refill_threshold > 0) ? (launch->refill_threshold < 32 ? launch->refill_threshold : 32) : 1;
-  a.grid = sm_count_of(device) * ((launch && launch->blocks_per_sm > 0 && launch->blocks_per_sm < occ) ? launch->blocks_per_sm : occ);
-  a.block = vs[idx].block;
-  e = vs[idx].run(a, s);
+  a.refill_threshold = shape.refill;
+  a.grid = shape.grid;
+  a.block = shape.v->block;
+  e = shape.v->run(a, s);
   if (e != cudaSuccess) return fail(KRR_ERR_CUDA, "persistent kernel launch: %s", cudaGetErrorString(e));
   krr::Queue q;
   std::memset(&q, 0, sizeof(q));

@@ -142,7 +142,8 @@ class ImageSpec:
 
 @dataclass(frozen=True)
 class LaunchConfig:
-    """Launch shape of the persistent kernel (0 = library default)."""
+    """Launch shape of the persistent kernel. With ``blocks_per_sm``, ``refill_threshold`` and
+    ``variant`` all 0 the library chooses the three for the number of photons."""
 
     block: int = 0            # threads per block of the plain kernel
     blocks_per_sm: int = 0    # resident blocks per SM (0 = as many as fit)
