@@ -96,7 +96,7 @@ struct Refs {
 template <class M>
 __device__ __forceinline__ double drift(double x, double den) {
   if constexpr (M::kFused) return x * den;
-  else return x / den;
+  else return quotient_any(x, den);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -138,8 +138,9 @@ struct Trig {
 };
 
 // Reference operation order (numba_kernel.py:111-197).  W is the working type; the metric is
-// always FP64 and cast to W before it meets the momenta.
-template <class W>
+// always FP64 and cast to W before it meets the momenta.  ROLLED: the step's stages as a loop
+// (dp_stages_loop), for kernels that keep many warps on an SM.
+template <class W, bool ROLLED = false>
 struct RefMode {
   using S = W;       // state type
   using K = W;       // stage type
@@ -148,6 +149,7 @@ struct RefMode {
   static constexpr bool kSaturate = false;
   static constexpr bool kMixed = false;
   static constexpr bool kFused = false;
+  static constexpr bool kRolled = ROLLED;
 
   __device__ static Trig accept_trig(double, const Trig& tr) { return tr; }
 
@@ -164,7 +166,7 @@ struct RefMode {
   __device__ static void stage(const Params& P, const R& ry, K h, const K acc[NV], K f[NV], Trig& tr, S yn[NV]) {
     S ys[NV];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) ys[i] = upd<RefMode<W>>(ry.y[i], h, acc[i]);
+    for (int i = 0; i < NV; ++i) ys[i] = upd<RefMode>(ry.y[i], h, acc[i]);
     if constexpr (LAST) {
 #pragma unroll
       for (int i = 0; i < NV; ++i) yn[i] = ys[i];
@@ -223,14 +225,17 @@ struct RefMode {
     return t;
   }
 
-  // Any operands, by IEEE division.  Out of line, its result by value: the operands the fast
-  // path declines are rare (a trial stage next to r = 0, the horizon or the axis, or a fraction
-  // that begins with 16 ones: one denominator in 65536).
-  struct Quotients {
-    double g[15];
+  // Any operands: sines with their large-argument path, IEEE division.  Out of line, its result by
+  // value: what the branch-free path declines is rare (a trial stage next to r = 0, the horizon or
+  // the axis, or a fraction that begins with 16 ones: one denominator in 65536).
+  struct Metric {
+    double g[15], s, c;
   };
-  __device__ __noinline__ static Quotients quotients_ieee(Terms t) {
-    Quotients q;
+  __device__ __noinline__ static Metric metric_any(const Params& P, double r, double th) {
+    Metric q;
+    q.s = sin(th);
+    q.c = cos(th);
+    const Terms t = terms(P, r, q.s, q.c, sin(2.0 * th));
     q.g[0] = t.n0 / t.sd;
     q.g[1] = t.n1 / t.sd;
     q.g[2] = t.dlt / t.sig;
@@ -249,41 +254,47 @@ struct RefMode {
     return q;
   }
 
-  // The 15 terms.  The branch-free quotients hold their values while nothing overflows or
-  // underflows: with sin^2, Sigma and Sigma Delta in [2^-120, 2^120] and the mass and spin in
-  // [2^-60, 2^60] (or spin 0; P.div_ok) every denominator lies in [2^-480, 2^480], and every
-  // numerator is 0 or in [2^-700, 2^700] (products of at most six such factors; a difference that
-  // is not 0 is at least 2^-53 of its terms).
+  // The 15 terms, without a branch but the one to metric_any.  The branch-free quotients hold their
+  // values while nothing overflows or underflows: with sin^2, Sigma and Sigma Delta in
+  // [2^-120, 2^120] and the mass and spin in [2^-60, 2^60] (or spin 0; P.div_ok) every denominator
+  // lies in [2^-480, 2^480], and every numerator is 0 or in [2^-700, 2^700] (products of at most six
+  // such factors; a difference that is not 0 is at least 2^-53 of its terms).  The sines and the
+  // cosine are the compiler's, told that the angle is moderate: their branch to the reduction of
+  // large arguments is then left out, and the same values come without it (a 64^2 image 2.35 ->
+  // 2.22 ms with the accepted steps' three divisions branch-free as well).
   __device__ static void metric(const Params& P, double r, double th, double g[15], Trig& tr) {
-    const double s = sin(th);
-    const double c = cos(th);
+    const bool near = fabs(th) < 1000.0;
+    const double x = near ? th : 0.0, x2 = 2.0 * x;
+    __builtin_assume(fabs(x) < 1000.0);
+    __builtin_assume(fabs(x2) < 2000.0);
+    const double s = sin(x), c = cos(x), sin2th = sin(x2);
     tr.s = s;
     tr.c = c;
-    const double sin2th = sin(2.0 * th);
     const Terms t = terms(P, r, s, c, sin2th);
     const unsigned gap = min(min(min(fraction_gap(t.sig), fraction_gap(t.sd)), min(fraction_gap(t.sd2), fraction_gap(t.sig2))),
                              min(min(fraction_gap(t.sds2), fraction_gap(t.sig2s2)), fraction_gap(t.sig2s4)));
-    if (gap != 0u && P.div_ok && moderate(t.s2) && moderate(t.sig) && moderate(t.sd)) {
-      const Recip i_sd = recip(t.sd), i_sig = recip(t.sig), i_sd2 = recip(t.sd2), i_sig2 = recip(t.sig2);
-      g[0] = quotient(t.n0, i_sd);
-      g[1] = quotient(t.n1, i_sd);
-      g[2] = quotient(t.dlt, i_sig);
-      g[3] = quotient_one(i_sig);
-      g[4] = quotient(t.n4, t.sds2);
-      g[5] = quotient(t.n5, i_sd2);
-      g[6] = quotient(t.n6, i_sd2);
-      g[7] = quotient(t.n7, i_sig2);
-      g[8] = quotient(t.n8, i_sig2);
-      g[9] = quotient(t.n8, t.sig2s2) + quotient(t.n9, i_sd2);
-      g[10] = quotient(t.n10, i_sd2);
-      g[11] = quotient(t.n11, i_sd2);
-      g[12] = quotient(t.n12, i_sig2);
-      g[13] = quotient(t.n13, i_sig2);
-      g[14] = quotient(t.n14, t.sig2s4) + quotient(t.m14, i_sd2);
-    } else {
-      const Quotients q = quotients_ieee(t);
+    const Recip i_sd = recip(t.sd), i_sig = recip(t.sig), i_sd2 = recip(t.sd2), i_sig2 = recip(t.sig2);
+    g[0] = quotient(t.n0, i_sd);
+    g[1] = quotient(t.n1, i_sd);
+    g[2] = quotient(t.dlt, i_sig);
+    g[3] = quotient_one(i_sig);
+    g[4] = quotient(t.n4, t.sds2);
+    g[5] = quotient(t.n5, i_sd2);
+    g[6] = quotient(t.n6, i_sd2);
+    g[7] = quotient(t.n7, i_sig2);
+    g[8] = quotient(t.n8, i_sig2);
+    g[9] = quotient(t.n8, t.sig2s2) + quotient(t.n9, i_sd2);
+    g[10] = quotient(t.n10, i_sd2);
+    g[11] = quotient(t.n11, i_sd2);
+    g[12] = quotient(t.n12, i_sig2);
+    g[13] = quotient(t.n13, i_sig2);
+    g[14] = quotient(t.n14, t.sig2s4) + quotient(t.m14, i_sd2);
+    if (!(near && gap != 0u && P.div_ok && moderate(t.s2) && moderate(t.sig) && moderate(t.sd))) {
+      const Metric q = metric_any(P, r, th);
 #pragma unroll
       for (int i = 0; i < 15; ++i) g[i] = q.g[i];
+      tr.s = q.s;
+      tr.c = q.c;
     }
   }
 
@@ -514,6 +525,7 @@ struct Fast64 {
   static constexpr bool kSaturate = false;
   static constexpr bool kMixed = false;
   static constexpr bool kFused = true;
+  static constexpr bool kRolled = false;
 
   __device__ static Trig accept_trig(double, const Trig& tr) { return tr; }
 
@@ -587,6 +599,7 @@ struct Mixed {
   // pipelines trace them again); MixedSat below rejects instead.
   static constexpr bool kSaturate = false;
   static constexpr bool kFused = true;
+  static constexpr bool kRolled = false;
 
   // FP32 copy of what the stages read: (r, r - r_plus), (p_r, p_theta) as packed pairs, theta
   // with its sine and cosine, and the ray's constants of motion.
@@ -799,7 +812,7 @@ __device__ __forceinline__ double carter(const Params& P, const Ray<M>& ry) {
   if constexpr (M::kFused) {
     if (lz != 0.0) lz2_over_s2 = (lz * lz) * rcp_newton<2>(s * s);
   } else {
-    if (lz != 0.0) lz2_over_s2 = (lz * lz) / (s * s);
+    if (lz != 0.0) lz2_over_s2 = quotient_any(lz * lz, s * s);
   }
   return p_th * p_th + (c * c) * (lz2_over_s2 - P.a2 * e * e);
 }
@@ -967,6 +980,98 @@ __device__ __forceinline__ void dp_stages_scalar(const Params& P, const Ray<M>& 
   }
 }
 
+// The Dormand-Prince stages of the rolled reference modes: one loop around a single copy of the
+// right-hand side.  Unrolled, its six copies make the step longer than the instruction cache holds:
+// with 8 warps per SM at different places of it, an instruction waited 2.1 to 2.6 cycles to be
+// fetched, of 6.0 in all; rolled 0.5, for 17 % more instructions (the values carried around the
+// loop).  With few warps the unrolled form is the faster, its neighbouring stages overlapping
+// (ref_variants).  Each pass computes its stage input from the last stage's value f and the sums
+// kept so far, by cases of the (uniform) stage number; the sums after k3 are begun as soon as it is
+// known and continued with each stage, in the reference's order of terms, so that k0, k1, k2 or
+// their successors are all that is held.  (Held in shared memory instead of registers: 12.0 ms
+// against 11.7 at 600^2.)
+template <class M>
+__device__ __forceinline__ void dp_stages_loop(const Params& P, const Ray<M>& ry, typename M::K h, typename M::K k6[NV],
+                                        typename M::S yn[NV], typename M::K esum[NV], Trig& tr) {
+  using K = typename M::K;
+  using S = typename M::S;
+  const K* k0 = ry.f;
+  auto c = [](double x) { return (K)x; };
+  // The right-hand side reads r, theta, p_r and p_theta only: the inner stages' sums leave out t and phi.
+  constexpr int IN[4] = {CR, CTH, CPR, CPTH};
+  K acc[4], f[NV], k1[4], u[NV];  // k1, then the last inner stage's sum; k2 in u, then the solution's sum
+  S ys[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) k1[i] = (K)0;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) f[i] = u[i] = esum[i] = (K)0;
+#pragma unroll 1
+  for (int st = 1; st <= 6; ++st) {
+    switch (st) {
+      case 1:
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = c(dp::A10) * k0[IN[q]];
+        break;
+      case 2:
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          k1[q] = f[IN[q]];
+          acc[q] = c(dp::A20) * k0[IN[q]] + c(dp::A21) * k1[q];
+        }
+        break;
+      case 3:
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          acc[q] = c(dp::A30) * k0[IN[q]] + c(dp::A31) * k1[q] + c(dp::A32) * f[IN[q]];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) u[i] = f[i];
+        break;
+      case 4:
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int i = IN[q];
+          acc[q] = c(dp::A40) * k0[i] + c(dp::A41) * k1[q] + c(dp::A42) * u[i] + c(dp::A43) * f[i];
+          k1[q] = c(dp::A50) * k0[i] + c(dp::A51) * k1[q] + c(dp::A52) * u[i] + c(dp::A53) * f[i];
+        }
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          esum[i] = c(dp::E0) * k0[i] + c(dp::E2) * u[i] + c(dp::E3) * f[i];
+          u[i] = c(dp::B0) * k0[i] + c(dp::B2) * u[i] + c(dp::B3) * f[i];
+        }
+        break;
+      case 5:
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = k1[q] + c(dp::A54) * f[IN[q]];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          u[i] = u[i] + c(dp::B4) * f[i];
+          esum[i] = esum[i] + c(dp::E4) * f[i];
+        }
+        break;
+      default:
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          u[i] = u[i] + c(dp::B5) * f[i];
+          esum[i] = esum[i] + c(dp::E5) * f[i];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = u[IN[q]];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ys[q] = upd<M>(ry.y[IN[q]], h, acc[q]);
+    M::rhs(P, ys[0], ys[1], ry.pt, ys[2], ys[3], ry.pph, f, tr);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) yn[IN[q]] = ys[q];
+  yn[CT] = upd<M>(ry.y[CT], h, u[CT]);
+  yn[CPH] = upd<M>(ry.y[CPH], h, u[CPH]);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    k6[i] = f[i];
+    esum[i] = esum[i] + c(dp::E6) * f[i];
+  }
+}
+
 // The mixed mode's stages on packed FP32 pairs.  sm_100 executes two FP32 multiply-adds in one
 // instruction (fma.rn.f32x2); with the components paired as (r, theta), (p_r, p_theta) and
 // (t, phi), each stage sum takes one packed operation per pair where the scalar form takes
@@ -1050,6 +1155,8 @@ __device__ __forceinline__ void dp_stages(const Params& P, const Ray<M>& ry, typ
   if constexpr (M::kMixed) {
     static_assert(!RK4, "the mixed mode integrates with Dormand-Prince 5(4) only");
     dp_stages_mixed<M>(P, ry, h, k6, yn, esum);
+  } else if constexpr (M::kRolled && !RK4) {
+    dp_stages_loop<M>(P, ry, h, k6, yn, esum, tr);
   } else {
     dp_stages_scalar<M, RK4>(P, ry, h, k6, yn, esum, tr, acc_rec);
   }

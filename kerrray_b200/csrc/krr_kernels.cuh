@@ -83,7 +83,7 @@ static __device__ __noinline__ double photon_start(const Image* __restrict__ ima
 // photon's image supplies the parameters and (when Y0 is null) the camera pixel.  index
 // (nullable) maps thread i to global photon index[i].
 template <class M, bool RK4>
-__global__ void k_trace_plain(Params P, const Image* __restrict__ images, int n_images,
+__global__ void k_trace_plain(const __grid_constant__ Params P, const Image* __restrict__ images, int n_images,
                               const double* __restrict__ Y0, const long long* __restrict__ index, long long n,
                               Outputs o, Queue* q) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -113,8 +113,10 @@ __global__ void k_trace_plain(Params P, const Image* __restrict__ images, int n_
   }
   if (q) {  // warp-aggregated counters (blockDim is a multiple of 32)
     constexpr unsigned FULL = 0xffffffffu;
+    unsigned long long longest = n_att;  // the warp's iterations
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
+      longest = max(longest, __shfl_down_sync(FULL, longest, off));
       n_att += __shfl_down_sync(FULL, n_att, off);
       n_acc += __shfl_down_sync(FULL, n_acc, off);
       n_ret += __shfl_down_sync(FULL, n_ret, off);
@@ -123,6 +125,8 @@ __global__ void k_trace_plain(Params P, const Image* __restrict__ images, int n_
       atomicAdd(&q->retired, n_ret);
       atomicAdd(&q->attempts, n_att);
       atomicAdd(&q->accepted, n_acc);
+      atomicAdd(&q->lane_iters, longest * 32ull);
+      atomicAdd(&q->busy_iters, n_att);
     }
   }
 }

@@ -79,4 +79,17 @@ __device__ __forceinline__ bool moderate(double x) {
   return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x38700000u < 0x0f000000u;
 }
 
+// a / b for any operands: branch-free in the range where that holds (|b| in [2^-400, 2^400], a 0 or
+// |a| in [2^-900, 2^900), which leaves |a / b| normal or its residual exact), else by IEEE division
+// out of line.
+static __device__ __noinline__ double quotient_ieee(double a, double b) { return a / b; }
+
+__device__ __forceinline__ double quotient_any(double a, double b) {
+  const unsigned ha = (unsigned)__double2hiint(a) & 0x7fffffffu, hb = (unsigned)__double2hiint(b) & 0x7fffffffu;
+  const double q = quotient(a, b);
+  const bool ok = hb - 0x26f00000u < 0x32000000u && fraction_gap(b) != 0u &&
+                  (a == 0.0 || ha - 0x07b00000u < 0x70800000u);
+  return ok ? q : quotient_ieee(a, b);
+}
+
 }  // namespace krr
