@@ -328,9 +328,9 @@ int check_precision(int32_t precision, const krr_options* o) {
   return KRR_OK;
 }
 
-cudaError_t launch_plain(int32_t precision, const krr_options* o, const krr::PlainArgs& a, cudaStream_t s) {
+// block: a multiple of 32 (the kernel's warp-aggregated counters assume it).
+cudaError_t launch_plain(int32_t precision, const krr_options* o, const krr::PlainArgs& a, int block, cudaStream_t s) {
   const bool rk4 = o->method == 1;
-  const int block = 128;  // a multiple of 32 (the kernel's warp-aggregated counters assume it)
   if (precision == KRR_PREC_REFERENCE) return krr::ref_plain(o->dtype == 1, rk4, a, block, s);
   return krr::fast_plain(precision == KRR_PREC_MIXED, rk4, a, block, s);
 }
@@ -451,19 +451,25 @@ const krr::Variant* variants_for(int32_t precision, const krr_options* o, int* c
 }
 
 // The launch shape a caller asked for or, with none of variant, blocks_per_sm and refill_threshold
-// set, the library's for `total` photons (each measured on the B200; the results never differ):
-// - a queue that fits the lanes of the shape without a register cap (variant 0: fast64 2 blocks of
-//   128 per SM, mixed 3, reference 2) is bound by its longest photon's chain of steps, and that
-//   shape has the shortest: 100^2 photons in fast64 0.69 ms against 0.78-0.83 at 12 warps per SM.
-//   It gets only the blocks it fills, so that no scheduler holds two warps while others idle:
-//   0.69 -> 0.57 ms, reference order 2.42 -> 2.06.
+// set, the library's for `total` photons (each measured on the B200; the results never differ).
+// With `lanes` the resident lanes of variant 0, the shape without a register cap:
+// - few photons per lane: one photon per thread, the block scheduler replacing a warp that ends. No
+//   queue, no refills (a photon's start costs its warp a step attempt or more): in fast64 10k photons
+//   0.52 ms against 0.60 from the queue, 147k photons of 36 images 3.9 against 4.2; mixed 0.41
+//   against 0.50 and, 98k photons, 2.5 against 3.2. At 5 photons per lane of a mixed set and more the
+//   queue wins (fast64, 737k photons of 72 images: 14.5 ms plain, 12.1 queue; one image: the same
+//   either way from 360k photons up), so up to 4 per lane in the fast modes. In reference order the
+//   queue's kernel is the rolled one, which pays off earlier: 40k photons 4.8 ms plain, 6.0 queue;
+//   90k 5.7 and 5.0: up to 1.5 per lane. Blocks of one warp spread best over the SMs, but up to 128
+//   photons per SM blocks of four, which put one warp on each scheduler: 10k photons in reference
+//   order 2.37 ms in blocks of 32, 2.14 of 128; 20k at rtol 1e-9 7.0 and 7.3.
+// - the queue on that few photons (where a re-trace needs it) takes variant 0, with the shortest
+//   chain per step, on only the blocks it fills: 100^2 in fast64 0.69 -> 0.57 ms.
 // - a longer queue is bound by throughput: variant 1 (fast64 168 registers, 12 warps per SM; mixed
-//   128, 16 warps), and idle lanes wait until several can be refilled together, since a photon's
-//   start costs its warp about as much as a step attempt (the reference order's more than one).
-//   12.4M photons in fast64 221 ms (variant 0, refilling at 1 idle lane), 188 (variant 1), 166.5
-//   (at 6); 172.9 at 2, 171.2 at 8. Mixed 1024^2 7.34 -> 5.91 ms. At 300^2 (90k photons, 2.4 per
-//   lane of variant 0) fast64 1.22 -> 1.07 ms, mixed the same either way. Reference order 600^2:
-//   21.4 ms at 1, 16.0 at 4, 14.3 at 8, 13.8 at 12 (300^2: 5.2, 4.8, 4.6, 4.6).
+//   128, 16 warps; reference the rolled stages), and idle lanes wait until several are refilled
+//   together. 12.4M photons in fast64 221 ms (variant 0, refilling at 1 idle lane), 188 (variant 1),
+//   166.5 (at 6); 172.9 at 2, 171.2 at 8. Mixed 1024^2 7.34 -> 5.91 ms. Reference order 600^2,
+//   unrolled: 21.4 ms at 1, 16.0 at 4, 14.3 at 8, 13.8 at 12 (300^2: 5.2, 4.8, 4.6, 4.6).
 int persistent_shape(int device, int32_t precision, const krr_options* o, const krr_launch* l, long long total,
                      LaunchShape& s) {
   int count = 0;
@@ -475,8 +481,12 @@ int persistent_shape(int device, int32_t precision, const krr_options* o, const 
   const long long sms = sm_count_of(device);
   int occ = vs[idx].occupancy();
   bool fits = true;
+  s.plain_block = 0;
   if (!chosen) {
-    fits = total <= sms * std::max(occ, 0) * vs[0].block;
+    const long long lanes = sms * std::max(occ, 0) * vs[0].block;
+    fits = total <= lanes;
+    if (total <= (precision == KRR_PREC_REFERENCE ? lanes + lanes / 2 : 4 * lanes))
+      s.plain_block = total <= sms * 128 ? 128 : 32;
     if (!fits && count > 1) {
       idx = 1;
       occ = vs[idx].occupancy();
@@ -615,6 +625,10 @@ int prepare_pipeline(int device, const krr_image* images, int n_images, long lon
   LaunchShape shape{};
   rc = persistent_shape(device, precision, o0, launch, total, shape);
   if (rc) return rc;
+  if (shape.plain_block > 0 && !p.retrace && !p.plain) {
+    p.plain = true;
+    p.plain_block = shape.plain_block;
+  }
   p.main_v = shape.v;
   p.main.images = p.w.images;
   p.main.n_images = n_images;
@@ -1005,7 +1019,7 @@ int krr_integrate_batch_device(int device, double mass, double spin, const doubl
   a.n = n;
   a.o = to_outputs(d_out);
   a.q = nullptr;
-  KRR_CUDA(launch_plain(precision, options, a, static_cast<cudaStream_t>(stream)));
+  KRR_CUDA(launch_plain(precision, options, a, 32, static_cast<cudaStream_t>(stream)));
   return KRR_OK;
 }
 
@@ -1033,12 +1047,37 @@ int krr_integrate_batch(int device, double mass, double spin, const double* Y0, 
     krr_result dev;
     rc = device_results(c, n, out, options->disk_plane != 0, &dev);
     if (rc) return rc;
-    krr::PlainArgs a{};
-    a.P = make_params(mass, spin, options);
-    a.Y0 = d_Y0;
-    a.n = n;
-    a.o = to_outputs(&dev);
-    KRR_CUDA(launch_plain(precision, options, a, c->stream));
+    // One ray per thread or through the work queue, whichever is faster for n rays.
+    LaunchShape shape{};
+    rc = persistent_shape(device, precision, options, nullptr, n, shape);
+    if (rc) return rc;
+    if (shape.plain_block > 0) {
+      krr::PlainArgs a{};
+      a.P = make_params(mass, spin, options);
+      a.Y0 = d_Y0;
+      a.n = n;
+      a.o = to_outputs(&dev);
+      KRR_CUDA(launch_plain(precision, options, a, shape.plain_block, c->stream));
+    } else {
+      krr::Image im{};
+      im.P = make_params(mass, spin, options);
+      im.count = n;
+      KRR_CUDA(c->buf[B_QUEUE].ensure(work_bytes(1, 0)));
+      const WorkLayout w = work_layout(c->buf[B_QUEUE].p, 1, 0);
+      KRR_CUDA(cudaMemsetAsync(w.q0, 0, sizeof(krr::Queue), c->stream));
+      KRR_CUDA(cudaMemcpyAsync(w.images, &im, sizeof(im), cudaMemcpyHostToDevice, c->stream));
+      krr::PersistArgs a{};
+      a.images = w.images;
+      a.n_images = 1;
+      a.total = n;
+      a.Y0 = d_Y0;
+      a.o = to_outputs(&dev);
+      a.q = w.q0;
+      a.refill_threshold = shape.refill;
+      a.grid = shape.grid;
+      a.block = shape.v->block;
+      KRR_CUDA(shape.v->run(a, c->stream));
+    }
     rc = copy_results_back(c, n, &dev, out);
     if (rc) return rc;
     KRR_CUDA(cudaStreamSynchronize(c->stream));

@@ -19,10 +19,11 @@ krr::Outputs to_outputs(const krr_result* r);
 const krr::Variant* variants_for(int32_t precision, const krr_options* o, int* count);
 int sm_count_of(int device);
 
-// The persistent kernel's launch: compiled shape, blocks, idle lanes before a warp refills.
+// The persistent kernel's launch: compiled shape, blocks, idle lanes before a warp refills; and
+// whether one photon per thread in blocks of `plain_block` threads is the faster launch (0: no).
 struct LaunchShape {
   const krr::Variant* v;
-  int grid, refill;
+  int grid, refill, plain_block;
 };
 int persistent_shape(int device, int32_t precision, const krr_options* o, const krr_launch* l, long long total,
                      LaunchShape& s);
