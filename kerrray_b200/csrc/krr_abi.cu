@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <thread>
 #include <chrono>
 #include <climits>
@@ -19,6 +20,7 @@
 #include "../../include/kerrray_cuda.h"
 #include "krr_host.h"
 #include "krr_launch.h"
+#include "krr_staging.h"
 
 namespace krr_host {
 
@@ -214,6 +216,7 @@ struct Context {
   cudaEvent_t lens_fork = nullptr, lens_join = nullptr;
   int sm_count = 0;
   DevBuf buf[B_COUNT];
+  Staging staging;
 };
 
 std::mutex g_ctx_mu;
@@ -277,6 +280,15 @@ bool all_finite_parallel(const double* x, size_t n) {
   return std::all_of(ok.begin(), ok.end(), [](char v) { return v != 0; });
 }
 
+// Host doubles to the device on stream s, through the staging memory if they are pageable; *bad
+// (nullable) is set where a staged value is not finite.  The host array has been read on return,
+// unless it is pinned.
+int copy_in(Context* c, void* dst, const double* src, size_t bytes, cudaStream_t s, std::atomic<bool>* bad) {
+  if (host_pinned(src)) KRR_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+  else KRR_CUDA(c->staging.in(c->device, {{dst, src, bytes}}, s, bad));
+  return KRR_OK;
+}
+
 // Host Y0 (rows x 8) to the device buffer B_Y0, checked there for non-finite values before any
 // trace work (the reference raises on them).  The check runs on the device: a host scan of a
 // large sweep's Y0 (~1e8 doubles) took longer than the copy itself.  Waits for the stream.
@@ -285,7 +297,8 @@ int upload_y0(Context* c, const double* Y0, long long rows, const double** d_out
   KRR_CUDA(c->buf[B_Y0].ensure(bytes));
   KRR_CUDA(c->buf[B_FINITE].ensure(sizeof(unsigned long long)));
   auto* d_count = static_cast<unsigned long long*>(c->buf[B_FINITE].p);
-  KRR_CUDA(cudaMemcpyAsync(c->buf[B_Y0].p, Y0, bytes, cudaMemcpyHostToDevice, c->stream));
+  int rc = copy_in(c, c->buf[B_Y0].p, Y0, bytes, c->stream, nullptr);
+  if (rc) return rc;
   KRR_CUDA(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), c->stream));
   KRR_CUDA(krr::count_nonfinite(static_cast<const double*>(c->buf[B_Y0].p), rows * 8, d_count, c->sm_count, c->stream));
   unsigned long long bad = 0;
@@ -363,36 +376,34 @@ int device_results(Context* c, int64_t n, const krr_result* host, bool disk, krr
   return KRR_OK;
 }
 
-int copy_results_back(Context* c, int64_t n, const krr_result* dev, const krr_result* host) {
-  const size_t n8 = (size_t)n * 8 * sizeof(double), n1 = (size_t)n * sizeof(double);
-  struct Pair { void* dst; const void* src; size_t bytes; };
-  Pair pairs[] = {
-      {host->Y, dev->Y, n8}, {host->state, dev->state, n1}, {host->n_steps, dev->n_steps, n1},
-      {host->n_rejected, dev->n_rejected, n1}, {host->lam, dev->lam, n1},
-      {host->max_null_error, dev->max_null_error, n1}, {host->max_energy_drift, dev->max_energy_drift, n1},
-      {host->max_lz_drift, dev->max_lz_drift, n1}, {host->max_carter_drift, dev->max_carter_drift, n1},
-      {host->event_Y, dev->event_Y, n8}, {host->event_hit, dev->event_hit, (size_t)n},
-  };
-  for (auto& p : pairs)
-    if (p.dst && p.src && p.bytes) KRR_CUDA(cudaMemcpyAsync(p.dst, p.src, p.bytes, cudaMemcpyDeviceToHost, c->stream));
-  return KRR_OK;
-}
-
-// Rows [r0, r1) of every requested result, device to host, on stream s.
-int copy_rows_back(const krr_result* dev, const krr_result* host, long long r0, long long r1, cudaStream_t s) {
+// Rows [r0, r1) of every requested result as copies to the host: through the staging memory the
+// spans whose host array is pageable, directly the others.
+void result_spans(const krr_result* dev, const krr_result* host, long long r0, long long r1,
+                  std::vector<CopySpan>& staged, std::vector<CopySpan>& direct) {
   const size_t n = (size_t)(r1 - r0), o = (size_t)r0;
   struct Slice { void* dst; const void* src; size_t row; };
-  Slice sl[] = {
+  const Slice sl[] = {
       {host->Y, dev->Y, 64}, {host->state, dev->state, 8}, {host->n_steps, dev->n_steps, 8},
       {host->n_rejected, dev->n_rejected, 8}, {host->lam, dev->lam, 8}, {host->max_null_error, dev->max_null_error, 8},
       {host->max_energy_drift, dev->max_energy_drift, 8}, {host->max_lz_drift, dev->max_lz_drift, 8},
       {host->max_carter_drift, dev->max_carter_drift, 8}, {host->event_Y, dev->event_Y, 64},
       {host->event_hit, dev->event_hit, 1},
   };
-  for (auto& x : sl)
-    if (x.dst && x.src && n)
-      KRR_CUDA(cudaMemcpyAsync(static_cast<char*>(x.dst) + o * x.row, static_cast<const char*>(x.src) + o * x.row,
-                               n * x.row, cudaMemcpyDeviceToHost, s));
+  for (const auto& x : sl)
+    if (x.dst && x.src && n) {
+      const CopySpan c{static_cast<char*>(x.dst) + o * x.row, static_cast<const char*>(x.src) + o * x.row, n * x.row};
+      (host_pinned(x.dst) ? direct : staged).push_back(c);
+    }
+}
+
+// Those rows, device to host, on stream s; every byte is in place on return.
+int copy_rows_back(Context* c, const krr_result* dev, const krr_result* host, long long r0, long long r1,
+                   cudaStream_t s) {
+  std::vector<CopySpan> staged, direct;
+  result_spans(dev, host, r0, r1, staged, direct);
+  for (const CopySpan& x : direct) KRR_CUDA(cudaMemcpyAsync(x.dst, x.src, x.bytes, cudaMemcpyDeviceToHost, s));
+  if (!staged.empty()) KRR_CUDA(c->staging.out(c->device, staged, s));
+  KRR_CUDA(cudaStreamSynchronize(s));
   return KRR_OK;
 }
 
@@ -846,8 +857,9 @@ int run_images(Context* c, const krr_image* images, const std::vector<krr::Image
 // range's results copied to the host on a second stream while the next range is traced, and a
 // host Y0 copied in range by range on a third.  The copies (0.8 GB in, 1.6 GB out for the
 // 12.4M-photon sweep) then hide behind the trace except the first range's input and the last
-// range's output; each extra launch costs one tail of idle lanes.
-constexpr long long kChunkPhotons = 2'000'000;  // ranges of at least this many photons
+// range's output; each extra launch costs one tail of idle lanes.  (2.9M photons of 72 images with
+// pageable arrays: 61 ms in one range, 49 ms in four of 0.7M; ranges from 0.4M the same.)
+constexpr long long kChunkPhotons = 700'000;  // ranges of at least this many photons
 
 int run_images_overlapped(Context* c, const krr_image* images, const std::vector<krr::Image>& ims, long long total,
                           const double* host_Y0, const krr_launch* launch, const krr_result* d_out,
@@ -872,21 +884,25 @@ int run_images_overlapped(Context* c, const krr_image* images, const std::vector
     bound[k] = (k == chunks) ? total : total * acc / wsum;
     if (k < chunks) acc += wts[k];
   }
-  // A host Y0 goes up range by range on its own stream.  The host checks it (every value
-  // finite) while the ranges are traced, and a non-finite value fails the call before any result
-  // is copied out: such a photon ends as a NUMERICAL_FAILURE at its first classification, so the
-  // traces it reaches only run to completion.  (Checked before the launches, the scan of a
-  // large sweep's Y0 held back the first trace by ~10 ms.)
+  // A host Y0 goes up range by range on its own stream, each range's trace queued behind it.  The
+  // host checks it (every value finite) while the ranges are traced, and a non-finite value fails
+  // the call before any result is copied out: such a photon ends as a NUMERICAL_FAILURE at its
+  // first classification, so the traces it reaches only run to completion.  (Checked before the
+  // launches, the scan of a large sweep's Y0 held back the first trace by ~10 ms.)  A pageable Y0
+  // is checked as it passes through the staging memory.
   const double* d_Y0 = nullptr;
+  const bool y0_pinned = host_Y0 && host_pinned(host_Y0);
+  std::atomic<bool> bad{false};
+  auto upload = [&](int k) -> int {
+    const size_t off = (size_t)bound[k] * 8, n = (size_t)(bound[k + 1] - bound[k]) * 8;
+    int rc = copy_in(c, static_cast<double*>(c->buf[B_Y0].p) + off, host_Y0 + off, n * sizeof(double), c->h2d_stream, &bad);
+    if (rc) return rc;
+    KRR_CUDA(cudaEventRecord(c->h2d_ev[k], c->h2d_stream));
+    return KRR_OK;
+  };
   if (host_Y0) {
     KRR_CUDA(c->buf[B_Y0].ensure((size_t)total * 8 * sizeof(double)));
-    double* dst = static_cast<double*>(c->buf[B_Y0].p);
-    for (int k = 0; k < chunks; ++k) {
-      const size_t off = (size_t)bound[k] * 8, n = (size_t)(bound[k + 1] - bound[k]) * 8;
-      KRR_CUDA(cudaMemcpyAsync(dst + off, host_Y0 + off, n * sizeof(double), cudaMemcpyHostToDevice, c->h2d_stream));
-      KRR_CUDA(cudaEventRecord(c->h2d_ev[k], c->h2d_stream));
-    }
-    d_Y0 = dst;
+    d_Y0 = static_cast<const double*>(c->buf[B_Y0].p);
   }
   Pipeline p;
   int rc = prepare_pipeline(c->device, images, (int)ims.size(), total, d_Y0, launch, d_out, d_work, work_size, p);
@@ -913,19 +929,25 @@ int run_images_overlapped(Context* c, const krr_image* images, const std::vector
     krr::PersistArgs a = p.main;
     a.q = qs[k];
     a.total = bound[k + 1];
-    if (host_Y0) KRR_CUDA(cudaStreamWaitEvent(st, c->h2d_ev[k], 0));
+    if (host_Y0) {
+      rc = upload(k);
+      if (rc) return rc;
+      KRR_CUDA(cudaStreamWaitEvent(st, c->h2d_ev[k], 0));
+    }
     KRR_CUDA(p.main_v->run(a, st));
     KRR_CUDA(cudaEventRecord(c->chunk_ev[k], st));
   }
   for (int k = 1; k < chunks; k += 2) KRR_CUDA(cudaStreamWaitEvent(s, c->chunk_ev[k], 0));
   KRR_CUDA(cudaEventRecord(c->ev1, s));
-  if (host_Y0 && !all_finite_parallel(host_Y0, (size_t)total * 8)) return fail(KRR_ERR_INVALID, "Y0 must be finite");
-  // Every launch is queued before the first copy-out: a copy into pageable host memory returns
-  // only when it has finished, and must not hold back the next range's launch.
+  if (bad.load() || (y0_pinned && !all_finite_parallel(host_Y0, (size_t)total * 8)))
+    return fail(KRR_ERR_INVALID, "Y0 must be finite");
+  // Every launch is queued before the first copy-out, which returns only when it has finished.
   for (int k = 0; k < chunks; ++k) {
     KRR_CUDA(cudaStreamWaitEvent(c->copy_stream, c->chunk_ev[k], 0));
-    rc = copy_rows_back(d_out, host_out, bound[k], bound[k + 1], c->copy_stream);
-    if (rc) return rc;
+    std::vector<CopySpan> staged, direct;
+    result_spans(d_out, host_out, bound[k], bound[k + 1], staged, direct);
+    for (const CopySpan& x : direct) KRR_CUDA(cudaMemcpyAsync(x.dst, x.src, x.bytes, cudaMemcpyDeviceToHost, c->copy_stream));
+    if (!staged.empty()) KRR_CUDA(c->staging.out(c->device, staged, c->copy_stream));
   }
   krr::Queue q[4];
   std::memset(q, 0, sizeof(q));
@@ -1034,7 +1056,8 @@ int krr_integrate_batch(int device, double mass, double spin, const double* Y0, 
   if (rc) return rc;
   if (n < 0) return fail(KRR_ERR_INVALID, "n must be >= 0, got %lld", (long long)n);
   if (!out || (n > 0 && (!Y0 || !out->Y || !out->state))) return fail(KRR_ERR_INVALID, "Y0, Y and state must not be NULL");
-  if (n > 0 && !all_finite(Y0, (size_t)n * 8)) return fail(KRR_ERR_INVALID, "Y0 must be finite");
+  // Before the device is looked for, as the reference's check comes before its backend's work.
+  if (n > 0 && !all_finite_parallel(Y0, (size_t)n * 8)) return fail(KRR_ERR_INVALID, "Y0 must be finite");
   Context* c = nullptr;
   rc = get_context(device, &c);
   if (rc) return rc;
@@ -1042,7 +1065,8 @@ int krr_integrate_batch(int device, double mass, double spin, const double* Y0, 
   KRR_CUDA(cudaSetDevice(device));
   if (n > 0) {
     KRR_CUDA(c->buf[B_Y0].ensure((size_t)n * 8 * sizeof(double)));
-    KRR_CUDA(cudaMemcpyAsync(c->buf[B_Y0].p, Y0, (size_t)n * 8 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    rc = copy_in(c, c->buf[B_Y0].p, Y0, (size_t)n * 8 * sizeof(double), c->stream, nullptr);
+    if (rc) return rc;
     const double* d_Y0 = static_cast<const double*>(c->buf[B_Y0].p);
     krr_result dev;
     rc = device_results(c, n, out, options->disk_plane != 0, &dev);
@@ -1078,9 +1102,8 @@ int krr_integrate_batch(int device, double mass, double spin, const double* Y0, 
       a.block = shape.v->block;
       KRR_CUDA(shape.v->run(a, c->stream));
     }
-    rc = copy_results_back(c, n, &dev, out);
+    rc = copy_rows_back(c, &dev, out, 0, n, c->stream);
     if (rc) return rc;
-    KRR_CUDA(cudaStreamSynchronize(c->stream));
   }
   if (runtime_s) runtime_s[0] = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   return KRR_OK;
@@ -1184,8 +1207,11 @@ int krr_camera_states(int device, double mass, double spin, const krr_camera* ca
                               static_cast<int*>(c->buf[B_ERR].p), c->stream));
   int err = 0;
   KRR_CUDA(cudaMemcpyAsync(&err, c->buf[B_ERR].p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  KRR_CUDA(cudaMemcpyAsync(Y0, c->buf[B_Y0].p, (size_t)rows * 8 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  KRR_CUDA(cudaStreamSynchronize(c->stream));
+  krr_result host{}, dev{};
+  host.Y = Y0;
+  dev.Y = static_cast<double*>(c->buf[B_Y0].p);
+  rc = copy_rows_back(c, &dev, &host, 0, rows, c->stream);
+  if (rc) return rc;
   if (err) return fail(KRR_ERR_NOT_NULL, "tetrad projection is not null to 1e-10 (or no null momentum exists)");
   return KRR_OK;
 }
@@ -1632,10 +1658,7 @@ int krr_trace_images(int device, const krr_image* images, int32_t n_images, cons
     return run_images_overlapped(c, images, ims, total, Y0, launch, &dev, out, c->buf[B_QUEUE].p, wbytes, stats);
   rc = run_images(c, images, ims, total, d_Y0, launch, &dev, c->buf[B_QUEUE].p, wbytes, c->stream, stats);
   if (rc) return rc;
-  rc = copy_results_back(c, total, &dev, out);
-  if (rc) return rc;
-  KRR_CUDA(cudaStreamSynchronize(c->stream));
-  return KRR_OK;
+  return copy_rows_back(c, &dev, out, 0, total, c->stream);
 }
 
 }  // extern "C"
