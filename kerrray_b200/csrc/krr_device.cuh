@@ -135,12 +135,21 @@ __device__ __forceinline__ typename M::S upd(typename M::S y, typename M::K h, t
 // Carter constant (same function, same argument, so the same values the reference recomputes).
 struct Trig {
   double s, c;
+  bool ok;  // RefMode's unrolled stages: every evaluation so far was within the branch-free path
 };
 
 // Reference operation order (numba_kernel.py:111-197).  W is the working type; the metric is
-// always FP64 and cast to W before it meets the momenta.  ROLLED: the step's stages as a loop
-// (dp_stages_loop), for kernels that keep many warps on an SM.
-template <class W, bool ROLLED = false>
+// always FP64 and cast to W before it meets the momenta.  The step's stages are
+//   UNROLLED  without a branch from the first to the last, so that the compiler overlaps a stage's
+//             long quotients (of p_r and p_theta) with the next one's sines and denominators, whose
+//             r and theta are known early (a 64^2 image 1.91 ms of kernel with a way out at each
+//             evaluation, 1.82 without); an evaluation outside the branch-free path sends the
+//             whole step to the CAREFUL form, out of line (dp_stages);
+//   ROLLED    a loop (dp_stages_loop), for kernels that keep many warps on an SM;
+//   CAREFUL   any operands, each evaluation with its own way out.
+enum class Stages { UNROLLED, ROLLED, CAREFUL };
+
+template <class W, Stages FORM = Stages::UNROLLED>
 struct RefMode {
   using S = W;       // state type
   using K = W;       // stage type
@@ -149,7 +158,7 @@ struct RefMode {
   static constexpr bool kSaturate = false;
   static constexpr bool kMixed = false;
   static constexpr bool kFused = false;
-  static constexpr bool kRolled = ROLLED;
+  static constexpr bool kRolled = FORM == Stages::ROLLED, kStraight = FORM == Stages::UNROLLED;
 
   __device__ static Trig accept_trig(double, const Trig& tr) { return tr; }
 
@@ -171,7 +180,7 @@ struct RefMode {
 #pragma unroll
       for (int i = 0; i < NV; ++i) yn[i] = ys[i];
     }
-    rhs(P, ys[CR], ys[CTH], ry.pt, ys[CPR], ys[CPTH], ry.pph, f, tr);
+    rhs<kStraight>(P, ys[CR], ys[CTH], ry.pt, ys[CPR], ys[CPTH], ry.pph, f, tr);
   }
 
   // The 15 metric terms' numerators and denominators in the reference's order.
@@ -227,7 +236,7 @@ struct RefMode {
 
   // Any operands: sines with their large-argument path, IEEE division.  Out of line, its result by
   // value: what the branch-free path declines is rare (a trial stage next to r = 0, the horizon or
-  // the axis, or a fraction that begins with 16 ones: one denominator in 65536).
+  // the axis, or a fraction that begins with 20 ones: one denominator in 1,048,576).
   struct Metric {
     double g[15], s, c;
   };
@@ -254,7 +263,7 @@ struct RefMode {
     return q;
   }
 
-  // The 15 terms, without a branch but the one to metric_any.  The branch-free quotients hold their
+  // The 15 terms without a branch.  The branch-free quotients hold their
   // values while nothing overflows or underflows: with sin^2, Sigma and Sigma Delta in
   // [2^-120, 2^120] and the mass and spin in [2^-60, 2^60] (or spin 0; P.div_ok) every denominator
   // lies in [2^-480, 2^480], and every numerator is 0 or in [2^-700, 2^700] (products of at most six
@@ -262,7 +271,8 @@ struct RefMode {
   // cosine are the compiler's, told that the angle is moderate: their branch to the reduction of
   // large arguments is then left out, and the same values come without it (a 64^2 image 2.35 ->
   // 2.22 ms with the accepted steps' three divisions branch-free as well).
-  __device__ static void metric(const Params& P, double r, double th, double g[15], Trig& tr) {
+  // False, with values that must not be used, where that does not hold.
+  __device__ __forceinline__ static bool metric_straight(const Params& P, double r, double th, double g[15], Trig& tr) {
     const bool near = fabs(th) < 1000.0;
     const double x = near ? th : 0.0, x2 = 2.0 * x;
     __builtin_assume(fabs(x) < 1000.0);
@@ -289,19 +299,24 @@ struct RefMode {
     g[12] = quotient(t.n12, i_sig2);
     g[13] = quotient(t.n13, i_sig2);
     g[14] = quotient(t.n14, t.sig2s4) + quotient(t.m14, i_sd2);
-    if (!(near && gap != 0u && P.div_ok && moderate(t.s2) && moderate(t.sig) && moderate(t.sd))) {
-      const Metric q = metric_any(P, r, th);
+    return near && gap != 0u && P.div_ok && moderate(t.s2) && moderate(t.sig) && moderate(t.sd);
+  }
+
+  // f (6 integrated components) at state (r, th, pr, pth) with constants (pt, pph).  STRAIGHT: tr.ok
+  // is cleared where the values must not be used.
+  template <bool STRAIGHT = false>
+  __device__ static void rhs(const Params& P, S r, S th, S pt, S pr, S pth, S pph, K f[NV], Trig& tr) {
+    double g64[15];
+    const bool ok = metric_straight(P, (double)r, (double)th, g64, tr);
+    if constexpr (STRAIGHT) {
+      tr.ok = tr.ok && ok;
+    } else if (!ok) {
+      const Metric q = metric_any(P, (double)r, (double)th);
 #pragma unroll
-      for (int i = 0; i < 15; ++i) g[i] = q.g[i];
+      for (int i = 0; i < 15; ++i) g64[i] = q.g[i];
       tr.s = q.s;
       tr.c = q.c;
     }
-  }
-
-  // f (6 integrated components) at state (r, th, pr, pth) with constants (pt, pph).
-  __device__ static void rhs(const Params& P, S r, S th, S pt, S pr, S pth, S pph, K f[NV], Trig& tr) {
-    double g64[15];
-    metric(P, (double)r, (double)th, g64, tr);
     W g[15];
 #pragma unroll
     for (int i = 0; i < 15; ++i) g[i] = (W)g64[i];
@@ -525,7 +540,7 @@ struct Fast64 {
   static constexpr bool kSaturate = false;
   static constexpr bool kMixed = false;
   static constexpr bool kFused = true;
-  static constexpr bool kRolled = false;
+  static constexpr bool kRolled = false, kStraight = false;
 
   __device__ static Trig accept_trig(double, const Trig& tr) { return tr; }
 
@@ -599,7 +614,7 @@ struct Mixed {
   // pipelines trace them again); MixedSat below rejects instead.
   static constexpr bool kSaturate = false;
   static constexpr bool kFused = true;
-  static constexpr bool kRolled = false;
+  static constexpr bool kRolled = false, kStraight = false;
 
   // FP32 copy of what the stages read: (r, r - r_plus), (p_r, p_theta) as packed pairs, theta
   // with its sine and cosine, and the ray's constants of motion.
@@ -1148,6 +1163,35 @@ __device__ __forceinline__ void dp_stages_mixed(const Params& P, const Ray<M>& r
   esum[CPH] = es[2].y;
 }
 
+// The step of a RefMode for any operands, out of line with its operands and results by value.
+template <class M>
+struct StepStart {
+  typename M::S y[NV], pt, pph;
+  typename M::K f[NV], h;
+};
+template <class M>
+struct StepEnd {
+  typename M::K k6[NV], esum[NV];
+  typename M::S yn[NV];
+  Trig tr;
+};
+template <class M, bool RK4>
+static __device__ __noinline__ StepEnd<M> dp_stages_careful(const Params& P, StepStart<M> a) {
+  using C = RefMode<typename M::S, Stages::CAREFUL>;
+  Ray<C> ry;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    ry.y[i] = a.y[i];
+    ry.f[i] = a.f[i];
+  }
+  ry.pt = a.pt;
+  ry.pph = a.pph;
+  StepEnd<M> e;
+  if constexpr (RK4) dp_stages_scalar<C, true>(P, ry, a.h, e.k6, e.yn, e.esum, e.tr);
+  else dp_stages_loop<C>(P, ry, a.h, e.k6, e.yn, e.esum, e.tr);
+  return e;
+}
+
 template <class M, bool RK4>
 __device__ __forceinline__ void dp_stages(const Params& P, const Ray<M>& ry, typename M::K h, typename M::K k6[NV],
                                           typename M::S yn[NV], typename M::K esum[NV], Trig& tr,
@@ -1157,6 +1201,28 @@ __device__ __forceinline__ void dp_stages(const Params& P, const Ray<M>& ry, typ
     dp_stages_mixed<M>(P, ry, h, k6, yn, esum);
   } else if constexpr (M::kRolled && !RK4) {
     dp_stages_loop<M>(P, ry, h, k6, yn, esum, tr);
+  } else if constexpr (M::kStraight) {
+    tr.ok = true;
+    dp_stages_scalar<M, RK4>(P, ry, h, k6, yn, esum, tr);
+    if (!tr.ok) {
+      StepStart<M> a;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        a.y[i] = ry.y[i];
+        a.f[i] = ry.f[i];
+      }
+      a.pt = ry.pt;
+      a.pph = ry.pph;
+      a.h = h;
+      const StepEnd<M> e = dp_stages_careful<M, RK4>(P, a);
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        k6[i] = e.k6[i];
+        yn[i] = e.yn[i];
+        esum[i] = e.esum[i];
+      }
+      tr = e.tr;
+    }
   } else {
     dp_stages_scalar<M, RK4>(P, ry, h, k6, yn, esum, tr, acc_rec);
   }

@@ -10,21 +10,21 @@
 // bit for bit (for b as below and no overflow or underflow on the way; the callers check):
 //
 //   y   1/b by two Newton steps from the hardware reciprocal.  That is within a relative 2^-19 of
-//       1/b, so y before its last rounding is within 2^-76 and |y - 1/b| <= (1/2 + 2^-20) ulp(y);
-//   q0  within (1/2 + 2^-40) ulp of a/b: a (y + lo) with lo = (1 - b y) y, or RN(a y) corrected
+//       1/b (2^-19.9 over all 2^20 upper words of a fraction), so y before its last rounding is
+//       within 2^-76 and |y - 1/b| <= (1/2 + 2^-23) ulp(y);
+//   q0  within (1/2 + 2^-51) ulp of a/b: a (y + lo) with lo = (1 - b y) y, or RN(a y) corrected
 //       once by its residual;
 //   r   a - b q0, exact (a multiple of ulp(b) ulp(q0), at most 2^53 of them);
 //   q   RN(q0 + r y): before its rounding it differs from a/b by |a/b - q0| |1 - b y|.
 //
 // Scale a and b to [1, 2) and let u be the quotient's ulp.  Every rounding boundary m of the
 // quotient is a multiple of u/2, so a - b m, which is not zero, is at least ulp(b) u / 2 and a/b
-// lies u / (2^53 b) or more from m.  The difference above is at most (1/2 + 2^-40) u times
-// b (1/2 + 2^-20) 2^-53 (ulp(y) = 2^-53 for 1/b in (1/2, 1]).  It is the smaller of the two, and q
-// therefore RN(a/b), if b^2 < 4 (1 - 2^-18): for every b whose fraction does not begin with 20
-// ones, b < 2 - 2^-20 + 2^-32.  (b^2 < 4 - 2^-18 there, against the needed 4 - 2^-17 at worst, so
-// the test below asks for one zero among the first 16 bits.)  A zero numerator gives +0 whatever
-// its sign.  The last step, correcting a nearly correct quotient by its exact residual, is
-// Markstein's (IBM J. Res. Dev. 34 (1990) 111).
+// lies u / (2^53 b) or more from m.  The difference above is at most (1/2 + 2^-51) u times
+// b (1/2 + 2^-23) 2^-53 (ulp(y) = 2^-53 for 1/b in (1/2, 1]).  It is the smaller of the two, and q
+// therefore RN(a/b), if b^2 < 4 (1 - 2^-22 - 2^-49): for every b whose fraction does not begin with
+// 20 ones, b < 2 - 2^-20 and b^2 < 4 (1 - 2^-20 + 2^-42).  A zero numerator gives +0 whatever its
+// sign.  The last step, correcting a nearly correct quotient by its exact residual, is Markstein's
+// (IBM J. Res. Dev. 34 (1990) 111).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -68,10 +68,10 @@ __device__ __forceinline__ double quotient(double a, double b) {
   return fma(fma(-b, q1, a), y, q1);
 }
 
-// The test on a denominator's fraction, for several denominators by minima: 0 where the first 16
+// The test on a denominator's fraction, for several denominators by minima: 0 where the first 20
 // of its 52 bits are all ones.
 __device__ __forceinline__ unsigned fraction_gap(double b) {
-  return (~(unsigned)__double2hiint(b)) & 0x000ffff0u;
+  return (~(unsigned)__double2hiint(b)) & 0x000fffffu;
 }
 
 // Whether |x| lies in [2^-120, 2^120) (false for NaN and infinities).

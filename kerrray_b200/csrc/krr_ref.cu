@@ -19,10 +19,10 @@ cudaError_t ref_plain(bool dtype32, bool rk4, const PlainArgs& a, int block, cud
 // warps per SM without spills, 11.7 at 12 with, 13.0 at 16; 300^2 4.9, 4.4, 4.4, 4.7.
 const Variant* ref_variants(bool dtype32, bool rk4, int* count) {
   static const Variant v64[] = {make_variant<RefMode<double>, false, 128, 1>(),
-                                make_variant<RefMode<double, true>, false, 128, 3>()};
+                                make_variant<RefMode<double, Stages::ROLLED>, false, 128, 3>()};
   static const Variant v64rk4[] = {make_variant<RefMode<double>, true, 128, 1>()};
   static const Variant v32[] = {make_variant<RefMode<float>, false, 128, 1>(),
-                                make_variant<RefMode<float, true>, false, 128, 3>()};
+                                make_variant<RefMode<float, Stages::ROLLED>, false, 128, 3>()};
   static const Variant v32rk4[] = {make_variant<RefMode<float>, true, 128, 1>()};
   *count = rk4 ? 1 : 2;
   if (dtype32) return rk4 ? v32rk4 : v32;

@@ -48,7 +48,7 @@ def _denominators(rng: random.Random):
         yield rng.uniform(1.0, 2.0)
     for k in range(20):  # next to 1, and the largest fractions the kernels' test lets through
         yield 1.0 + k * 2.0**-52
-        yield 2.0 - 2.0**-16 - (k + 1) * 2.0**-52
+        yield 2.0 - 2.0**-20 - (k + 1) * 2.0**-52
     yield from (1.0, 1.5, math.sqrt(2.0))
 
 
