@@ -504,6 +504,7 @@ int persistent_shape(int device, int32_t precision, const krr_options* o, const 
     }
   }
   s.v = &vs[idx];
+  s.index = idx;
   if (occ < 1) return fail(KRR_ERR_CUDA, "persistent kernel variant %d cannot be resident on this device", idx);
   if (chosen) {
     const int bps = l->blocks_per_sm > 0 ? std::min(l->blocks_per_sm, occ) : occ;
@@ -676,7 +677,13 @@ int prepare_pipeline(int device, const krr_image* images, int n_images, long lon
     const krr::Variant* wv = krr::ref_wide_variant();
     if (wv->occupancy() < 1) return fail(KRR_ERR_UNSUPPORTED, "the critical-set kernel cannot be resident");
     const int sms = std::max(sm_count_of(device), 2);
-    const int crit_sms = std::min(sms - 1, (launch && launch->critical_sms > 0) ? launch->critical_sms : std::max(2, sms / 37));
+    // Below about half a million photons the pipeline ends with the critical photons' chains, not
+    // with the main trace: they then get twice the SMs, with one warp on each scheduler (a 300^2
+    // image 2.65 -> 2.12 ms, 640^2 2.69 -> 2.46; 800^2 3.67 -> 3.73, so not there; four times the
+    // SMs 2.10, 2.58).
+    const bool wide = total <= 512 * 1024 && !(launch && launch->critical_sms > 0);
+    const int crit_sms = std::min(sms - 1, (launch && launch->critical_sms > 0) ? launch->critical_sms
+                                                                                : std::max(2, sms / 37 * (wide ? 2 : 1)));
     p.main.risk = p.w.risk;
     p.main.pdl = krr::PDL_WAIT;
     p.crit = p.main;
@@ -688,7 +695,7 @@ int prepare_pipeline(int device, const krr_image* images, int n_images, long lon
     p.crit.index = p.w.list;
     p.crit.d_total = &p.w.q1->flagged;
     p.crit.risk = nullptr;
-    p.crit.flags = krr::TRACE_SPREAD;
+    p.crit.flags = krr::TRACE_SPREAD | (wide ? krr::TRACE_ONE_PER_SCHEDULER : 0);
     p.crit.pdl = krr::PDL_TRIGGER | krr::PDL_STAMP;
     // Photons unlike their analytic class: after a mixed trace, rays an FP32 overflow ended
     // early, traced again with the overflow taken as a rejection (MixedSat); otherwise in FP64.
@@ -698,12 +705,23 @@ int prepare_pipeline(int device, const krr_image* images, int n_images, long lon
     p.fix_v = (precision == KRR_PREC_MIXED) ? krr::mixed_sat_variant() : &fv[0];
     if (p.fix_v->occupancy() < 1) return fail(KRR_ERR_UNSUPPORTED, "the re-trace kernel cannot be resident");
     p.fix = p.crit;
+    p.fix.flags = krr::TRACE_SPREAD;
     p.fix.q = p.w.q2;
     p.fix.grid = sms * p.fix_v->occupancy();
     p.fix.block = p.fix_v->block;
     p.fix.d_total = &p.w.q2->flagged;
     p.fix.pdl = 0;
-    if (precision == KRR_PREC_MIXED) p.fix.flags |= krr::TRACE_RESUME;  // continue where the overflow stopped it
+    if (precision == KRR_PREC_MIXED) {
+      p.fix.flags |= krr::TRACE_RESUME;  // continue where the overflow stopped it
+      // Up to 3M photons the main trace resumes those rays itself (1024^2 5.86 -> 5.61 ms, 800^2 4.01
+      // -> 3.67): its kernel is 2.5 % slower for it, so that 2048^2 takes 21.3 ms either way.
+      const krr::Variant* rv = krr::mixed_restart_variant(shape.index);
+      if (rv && total <= 3'000'000 && rv->occupancy() >= 1) {
+        p.main_v = rv;
+        p.main.grid = std::min(p.main.grid, sms * rv->occupancy());
+        p.main.flags |= krr::TRACE_RESTART;
+      }
+    }
     p.re = p.fix;
     p.re.flags = krr::TRACE_SPREAD;  // from the camera: the plain kernel's exact arithmetic
     p.re.q = p.w.q3;
@@ -817,12 +835,12 @@ int finish_pipeline(const Pipeline& p, cudaStream_t s, krr_stats* stats, cudaEve
     stats->lane_slots = q[0].lane_iters;
     stats->busy_slots = q[0].busy_iters;
     stats->kernel_ms = ms;
-    stats->retraced = crit ? q[1].flagged + q[2].flagged + q[3].flagged : (p.retrace ? q[0].flagged : 0);
+    stats->retraced = crit ? q[1].flagged + q[0].restarted + q[2].flagged + q[3].flagged : (p.retrace ? q[0].flagged : 0);
     stats->retrace_attempts = q[1].attempts + q[2].attempts + q[3].attempts;
     stats->retrace_ms = p.retrace ? ms2 : 0.0;
     stats->critical = crit ? q[1].flagged : 0;
     stats->critical_ms = ms_c;
-    stats->rechecked = crit ? q[2].flagged + q[3].flagged : 0;
+    stats->rechecked = crit ? q[0].restarted + q[2].flagged + q[3].flagged : 0;
     stats->near_edge = p.near ? q[4].flagged : 0;
     stats->near_edge_attempts = p.near ? q[4].attempts : 0;
   }

@@ -155,7 +155,7 @@ struct RefMode {
   using K = W;       // stage type
   using N = W;       // error-norm type
   using D = double;  // diagnostics (running maxima and their denominators)
-  static constexpr bool kSaturate = false;
+  static constexpr bool kSaturate = false, kRestart = false;
   static constexpr bool kMixed = false;
   static constexpr bool kFused = false;
   static constexpr bool kRolled = FORM == Stages::ROLLED, kStraight = FORM == Stages::UNROLLED;
@@ -537,7 +537,7 @@ struct Fast64 {
   using K = double;
   using N = double;
   using D = float;  // the drift maxima: FP64 values, kept to single precision
-  static constexpr bool kSaturate = false;
+  static constexpr bool kSaturate = false, kRestart = false;
   static constexpr bool kMixed = false;
   static constexpr bool kFused = true;
   static constexpr bool kRolled = false, kStraight = false;
@@ -612,7 +612,7 @@ struct Mixed {
   // factor because its error norm is huge.  This mode ends such a ray as a NUMERICAL_FAILURE
   // like the reference does on a non-finite step (a handful of rays per million; the
   // pipelines trace them again); MixedSat below rejects instead.
-  static constexpr bool kSaturate = false;
+  static constexpr bool kSaturate = false, kRestart = false;
   static constexpr bool kFused = true;
   static constexpr bool kRolled = false, kStraight = false;
 
@@ -725,6 +725,11 @@ struct Mixed {
 struct MixedSat : Mixed {
   static constexpr bool kSaturate = true;
 };
+// The mixed mode of the work-queue kernel: Mixed until Ray::saturate is set, then MixedSat
+// (k_trace_persistent's TRACE_RESTART).
+struct MixedQueue : Mixed {
+  static constexpr bool kRestart = true;
+};
 // ------------------------------------------------------------------------------------------
 // The state of one ray between step attempts.
 // ------------------------------------------------------------------------------------------
@@ -746,6 +751,7 @@ struct Ray {
   int n_steps, n_rej;
   int state;
   bool rejected_before;
+  bool saturate;  // MixedQueue: a non-finite error norm is a rejection (MixedSat), not the ray's end
 };
 
 template <class M>
@@ -866,6 +872,7 @@ __device__ __forceinline__ void ray_init(const Params& P, const double y0[8], do
   ry.n_steps = 0;
   ry.n_rej = 0;
   ry.rejected_before = false;
+  ry.saturate = false;
   ry.state = classify<M>(P, ry, false);
 }
 
@@ -1318,7 +1325,7 @@ __device__ __forceinline__ void attempt(const Params& P, Ray<M>& ry, double* __r
       // Full-state slots: 0 t, 1 r, 2 th, 3 ph, 4 p_t (0), 5 p_r, 6 p_th, 7 p_phi (0).
       const N total = ((q[CT] + q[CR]) + (q[CTH] + q[CPH])) + (q[CPR] + q[CPTH]);
       if constexpr (M::kFused) {
-        if (!M::kSaturate && !finite_(total)) {
+        if (!M::kSaturate && !(M::kRestart && ry.saturate) && !finite_(total)) {
           finite = false;
           accept = false;
         } else {

@@ -53,6 +53,12 @@ const Variant* near_wide_variant() {
   return &v;
 }
 
+// The shapes of mixed variants 0 and 1 with TRACE_RESTART; null for the others.
+const Variant* mixed_restart_variant(int index) {
+  static const Variant v[] = {make_variant<MixedQueue, false, 128, 1>(), make_variant<MixedQueue, false, 128, 4>()};
+  return index == 0 || index == 1 ? &v[index] : nullptr;
+}
+
 // The mixed re-trace of the few rays an FP32 overflow ended early (MixedSat: an overflowing
 // trial step is a rejection, as in FP64).
 const Variant* mixed_sat_variant() {

@@ -23,7 +23,7 @@ int sm_count_of(int device);
 // whether one photon per thread in blocks of `plain_block` threads is the faster launch (0: no).
 struct LaunchShape {
   const krr::Variant* v;
-  int grid, refill, plain_block;
+  int index, grid, refill, plain_block;
 };
 int persistent_shape(int device, int32_t precision, const krr_options* o, const krr_launch* l, long long total,
                      LaunchShape& s);

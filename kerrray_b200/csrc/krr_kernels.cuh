@@ -39,6 +39,7 @@ struct Queue {
   unsigned long long flagged;     // photons appended to the re-trace list
   unsigned long long t_first;     // globaltimer (ns) of the first block's start (PDL_STAMP), from ~0
   unsigned long long t_last;      // globaltimer (ns) of the last block's end (PDL_STAMP)
+  unsigned long long restarted;   // photons an FP32 overflow ended, traced on in place (TRACE_RESTART)
   unsigned long long speculative; // edge bisection: photons traced ahead of their bracket
   unsigned long long discarded;   // edge bisection: attempts of speculative photons not needed
 };
@@ -144,8 +145,16 @@ __global__ void k_trace_plain(const __grid_constant__ Params P, const Image* __r
 // TRACE_RESUME -- a photon continues from the result row already in the outputs (its last
 // accepted state, affine parameter, counters and drift maxima: a trace that an FP32 overflow
 // ended early) with the first step size, instead of starting again at the camera.
-// TRACE_SKIP_NEAR -- RISK_NEAR photons are skipped as well (the near-edge kernel traces them).
-enum : int { TRACE_SPREAD = 1, TRACE_RESUME = 2, TRACE_SKIP_NEAR = 4 };
+// TRACE_SKIP_NEAR -- RISK_NEAR photons are skipped as well (the near-edge kernel traces them);
+// TRACE_RESTART -- a mixed photon that ends as a NUMERICAL_FAILURE though its analytic class is
+// known (an FP32 overflow) goes on in its lane from the row just written, exactly as TRACE_RESUME
+// would resume it in a kernel of its own, with overflows taken as rejections from there on; should it
+// still end unlike its class, it is marked for the reference-order re-trace.  A kernel after the main
+// trace for these three photons of a 1024^2 image took 0.41 ms, the length of their remaining chains
+// with the rest of the GPU idle; traced on in place they end with the others.
+// TRACE_ONE_PER_SCHEDULER -- only the first four warps of a block take photons, the others leave: a
+// block that fills an SM's registers for a few long chains then runs one warp on each scheduler.
+enum : int { TRACE_SPREAD = 1, TRACE_RESUME = 2, TRACE_SKIP_NEAR = 4, TRACE_RESTART = 8, TRACE_ONE_PER_SCHEDULER = 16 };
 
 template <class M>
 __device__ __forceinline__ void resume_from_outputs(const Params& P, const Outputs& o, long long g, Ray<M>& ry) {
@@ -168,6 +177,24 @@ __device__ __forceinline__ void resume_from_outputs(const Params& P, const Outpu
   ry.state = classify<M>(P, ry, false);
 }
 
+// A photon's start and resumption out of line (TRACE_RESTART), by value: the step loop's photon
+// stays in registers.
+template <class M>
+static __device__ __noinline__ Ray<M> restarted_photon(const Image* __restrict__ images, int img,
+                                                       const double* __restrict__ Y0, Outputs o, long long g, Queue* q) {
+  Ray<M> ry;
+  double y0[8];
+  const double q0 = photon_start(images, img, Y0, g, y0, q);
+  ray_init<M>(images[img].P, y0, q0, ry);
+  resume_from_outputs<M>(images[img].P, o, g, ry);
+  ry.saturate = true;
+  return ry;
+}
+
+__device__ __forceinline__ bool unlike_class(int risk, int state) {
+  return (risk == RISK_CAPTURE && state != CAPTURED) || ((risk == RISK_ESCAPE || risk == RISK_NEAR) && state != ESCAPED);
+}
+
 template <class M, bool RK4, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB)
     k_trace_persistent(const Image* __restrict__ images, int n_images, long long total,
@@ -180,7 +207,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
   if (d_total) total = (long long)*d_total;
   int cap = 32;
   if (flags & TRACE_SPREAD) {
-    const long long warps = (long long)gridDim.x * (blockDim.x / 32);
+    const long long warps = (long long)gridDim.x * ((flags & TRACE_ONE_PER_SCHEDULER) ? 4 : blockDim.x / 32);
     cap = (int)min(32LL, max(1LL, (total + warps - 1) / warps));
   }
   const unsigned lane = threadIdx.x & 31u;
@@ -188,16 +215,21 @@ __global__ void __launch_bounds__(MAXT, MINB)
   Ray<M> ry;
   ry.state = FAILURE;
   bool active = false;
-  bool drained = false;
+  bool drained = (flags & TRACE_ONE_PER_SCHEDULER) && threadIdx.x >= 128;  // nothing to do
   long long g = -1;
   int img = 0;
+  ry.saturate = false;
   // Lane statistics, added when a photon retires (every busy lane slot is one step attempt).
   // 32-bit lane totals, flushed to the queue's 64-bit counters before they could wrap.
   unsigned my_attempts = 0, my_accepted = 0, my_iters = 0;
+  auto near_budget = [&]() {
+    return ry.lam > 0.99 * images[img].P.lambda_max || ry.n_steps > 0.99 * (double)images[img].P.max_steps;
+  };
   auto retire = [&]() {
     ray_store<M>(ry, o, g);
-    if (risk && (ry.lam > 0.99 * images[img].P.lambda_max || ry.n_steps > 0.99 * (double)images[img].P.max_steps))
-      risk[g] = RISK_RECHECK;
+    if (risk) {
+      if (M::kRestart && ry.saturate ? unlike_class(risk[g], ry.state) : near_budget()) risk[g] = RISK_RECHECK;
+    }
     const unsigned long long ra = (unsigned long long)ry.attempts;
     if (ra >= (1ull << 30) || my_attempts >= (1u << 30)) {
       atomicAdd(&q->attempts, ra + my_attempts);
@@ -257,6 +289,15 @@ __global__ void __launch_bounds__(MAXT, MINB)
       double* ev = o.event_Y ? o.event_Y + g * 8 : nullptr;
       unsigned char* hit = o.event_hit ? o.event_hit + g : nullptr;
       attempt<M, RK4>(im.P, ry, ev, hit);
+      if constexpr (M::kRestart) {
+        if (ry.state == FAILURE && (flags & TRACE_RESTART) && !ry.saturate && !near_budget() &&
+            unlike_class(risk[g], FAILURE)) {
+          ray_store<M>(ry, o, g);
+          my_attempts += (unsigned)ry.attempts;
+          ry = restarted_photon<M>(images, img, Y0, o, g, q);
+          atomicAdd(&q->restarted, 1ull);
+        }
+      }
       if (ry.state != RUNNING) {
         retire();
         active = false;

@@ -17,6 +17,7 @@ const Variant* ref_variants(bool dtype32, bool rk4, int* count);
 cudaError_t fast_plain(bool mixed, bool rk4, const PlainArgs& a, int block, cudaStream_t s);
 const Variant* fast_variants(bool mixed, bool rk4, int* count);
 const Variant* mixed_sat_variant();
+const Variant* mixed_restart_variant(int index);
 
 // theta and phi where each escaped ray (state ESCAPED) crosses r = r_s, flown back from its final
 // state Y; NaN for the other rows.
