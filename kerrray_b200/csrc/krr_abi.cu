@@ -1557,14 +1557,13 @@ int krr_bisect_edges(int device, const krr_edge_case* cases, int32_t n_cases, co
   std::lock_guard<std::mutex> lk(ctx->mu);
   KRR_CUDA(cudaSetDevice(device));
   // The items by the cost of their case, most expensive first (the DP5 step count grows like
-  // rtol^-1/5); the kernel deals them over its warps, so that every warp holds items of every
-  // tolerance and the cheap ones, ending early, lend their lanes to the expensive ones.  That
-  // needs the cases' parameters in shared memory (krr::edge_params_in_smem); with more cases the
-  // items keep their order, and a warp's lanes mostly share a case.
-  const bool deal = krr::edge_params_in_smem(n_cases);
+  // rtol^-1/5), so that the cheap ones make the launch's tail.  A warp's lanes then hold items of
+  // several cases, which needs the cases' parameters in shared memory (krr::edge_params_in_smem);
+  // with more cases the items keep their order, and a warp's lanes mostly share a case.
+  const bool by_case = krr::edge_params_in_smem(n_cases);
   std::vector<long long> order((size_t)n_items);
   for (int64_t i = 0; i < n_items; ++i) order[(size_t)i] = i;
-  if (deal) {
+  if (by_case) {
     std::vector<int> by_cost((size_t)n_cases);
     for (int k = 0; k < n_cases; ++k) by_cost[(size_t)k] = k;
     std::stable_sort(by_cost.begin(), by_cost.end(),
@@ -1612,13 +1611,11 @@ int krr_bisect_edges(int device, const krr_edge_case* cases, int32_t n_cases, co
   a.hi = d_hi;
   a.failures = d_fail;
   a.order = d_order;
-  a.deal = deal;
   a.star = d_star;
   a.n_cases = n_cases;
   a.n_items = n_items;
   a.iterations = iterations;
   a.q = d_q;
-  a.refill_threshold = 1;
   KRR_CUDA(cudaEventRecord(ctx->ev0, s));
   KRR_CUDA(krr::edge_predict(a, s));
   KRR_CUDA(precision == KRR_PREC_REFERENCE ? krr::ref_bisect(a, s) : krr::fast_bisect(precision == KRR_PREC_MIXED, a, s));

@@ -248,18 +248,17 @@ cudaError_t count_nonfinite(const double* x, long long n, unsigned long long* co
   return cudaGetLastError();
 }
 
-// The fast64 bisection at three blocks per SM (168 registers, spilling 44 B) only for a study
-// large enough to keep those lanes at most 3/4 of its items (run_bisect's rule); below that at
-// two blocks per SM, whose register budget holds the whole kernel (186-188 registers, no spills:
-// 2.5 % faster on the 51,840-item edge study).  On a study of 155,520 items the build for three
-// at three blocks per SM takes 283-288 ms, the build for two at two 310-318 ms.
+// The fast64 bisection: a study of up to four items per warp is bound by its items' chains and runs
+// the build for two blocks per SM (200 registers, no spills): 540 items 13.5 ms, 16.6 in the build
+// for three.  A longer one runs that (168 registers, spilling 44 B), its 12 warps per SM hiding more:
+// 8676 items 31.5 ms against 33 to 38, 51,840 items 100.5 against 106.
 cudaError_t fast_bisect(bool mixed, const EdgeArgs& a, cudaStream_t s) {
   if (mixed) return run_bisect<Mixed, 128, 1>(a, s);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (4LL * sms * 3 * 128 <= 3LL * a.n_items) return run_bisect<Fast64, 128, 3>(a, s);
-  return run_bisect<Fast64, 128, 2>(a, s);
+  const long long warps = 2LL * sms * (128 / 32);
+  return a.n_items <= 4 * warps ? run_bisect<Fast64, 128, 2>(a, s) : run_bisect<Fast64, 128, 3>(a, s);
 }
 
 }  // namespace krr

@@ -331,31 +331,32 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // traced; ESCAPED moves hi to mid, anything else moves lo to mid; a result that is neither
 // ESCAPED nor CAPTURED counts as a failure.
 //
-// One lane owns an item and runs its halvings one after another.  A warp takes at most
-// ceil(items / warps) items, so that a study smaller than the grid is spread over every warp, and
-// its other lanes trace ahead: a helper takes a node of the bisection tree below an owner's
-// current bracket, at some depth d (the bracket the item holds after the owner's photon and the
-// next d - 1 ones), and traces its midpoint while the owner's photon is still running.  When the
-// owner's photon ends, the helpers on the outcome's side move up one level; the one at depth 1
-// inherits the item and continues with its photon (possibly already ended, which settles one more
-// halving at once); the helpers on the other side are discarded.  Every midpoint is
-// 0.5 * (lo + hi) of the bracket the sequential bisection would hold there, so the results are the
-// sequential ones bit for bit.
+// One lane owns an item and runs its halvings one after another.  A warp takes a few items (a
+// quarter of an even share, at most EDGE_CAP), so that a study is spread over every warp, and its
+// other lanes trace ahead: a helper takes a node of the bisection tree below an owner's current
+// bracket, at some depth d (the bracket the item holds after the owner's photon and the next d - 1
+// ones), and traces its midpoint while the owner's photon is still running.  When the owner's photon
+// ends, the helpers on the outcome's side move up one level; the one at depth 1 inherits the item
+// and continues with its photon (possibly already ended, which settles one more halving at once);
+// the helpers on the other side are discarded.  Every midpoint is 0.5 * (lo + hi) of the bracket the
+// sequential bisection would hold there, so the results are the sequential ones bit for bit.
 //
 // Which nodes are worth tracing is predicted: k_edge_predict finds each item's analytic edge
 // radius `star` from the constants of motion, and a photon further than EDGE_CONF * rtol M from
 // it almost surely ends on its analytic side (the integration moves the edge by about 2 rtol M; a
 // bracket that no longer holds `star` widens the doubt).  The nodes along the predicted path, down
 // to the first photon closer than that (its length is the owner's `chain`: about 20 levels of a
-// 6 M bracket at rtol 1e-6, 31 at 1e-10), are traced first, then the tree below the path's end,
-// where either outcome is possible.  A wrong prediction costs the attempts of the nodes below it,
-// nothing else.
+// 6 M bracket at rtol 1e-6, 31 at 1e-10), are traced first; lanes that no path needs take further
+// items, most expensive first; and once the queue is drained, the tree below the paths' ends, where
+// either outcome is possible.  A wrong prediction costs the attempts of the nodes below it, nothing
+// else.
 //
 // Measured (kernel, B200).  One edge, 90 directions, 36 halvings, rtol 1e-6, reference order: 87 ms
 // with the first three warps holding every item, 20 ms now (2000 attempts per warp for 36 halvings
-// of 341 each).  12 cases x 241 directions x 3 tolerances, fast64: 110 -> 36 ms; with the items in
-// runs of one tolerance instead of dealt, 52 ms.  x 1440 directions (51,840 items, every lane an
-// owner until the queue is drained): 127 -> 116 ms.  EDGE_CONF 2 and 16 within 5 % of 4 on all three.
+// of 341 each).  12 cases x 241 directions x 3 tolerances, fast64: 110 -> 31 ms; with an even share of
+// the items per warp from the start (8 a warp, dealt so that each holds every tolerance) 36 ms.
+// x 1440 directions (51,840 items): 127 -> 100 ms, 115 with an even share.  EDGE_CONF 2 and 16 within
+// 5 % of 4 on all three.
 // ------------------------------------------------------------------------------------------
 struct EdgeCase {
   Params P;
@@ -372,13 +373,11 @@ struct EdgeArgs {
   double* hi;
   long long* failures;
   const long long* order;  // the items, most expensive first
-  bool deal;               // deal them over the warps (otherwise in order)
   double* star;            // predicted edge radius of each item (k_edge_predict)
   int n_cases;
   long long n_items;
   int iterations;
   Queue* q;
-  int refill_threshold;
   int grid, block;
 };
 
@@ -408,6 +407,8 @@ enum : int { EDGE_IDLE = 0, EDGE_OWNER = 1, EDGE_HELPER = 2 };
 // traced EDGE_DEPTH levels deep, its node t levels below the end with path bits p being bit
 // (2^t - 2 + p) of a 32-bit mask.
 constexpr int EDGE_DEPTH = 4, EDGE_CHAIN = 31;
+// Items a warp holds before its lanes turn to the predicted paths: a quarter of an even share, at most 4.
+constexpr int EDGE_SPLIT = 4, EDGE_CAP = 4;
 constexpr double EDGE_CONF = 4.0;  // of rtol M: nearer to the predicted edge, either outcome is possible
 constexpr double EDGE_OFF = 3.0;   // of the least error of the prediction that the bracket shows
 __device__ __forceinline__ int edge_node(int d, unsigned p) { return (1 << d) - 2 + (int)p; }
@@ -456,17 +457,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
   int role = EDGE_IDLE, host = 0, depth = 0;
   unsigned path = 0;
   const long long warps = (long long)gridDim.x * (MAXT / 32);
-  const int cap = (int)min(32LL, (a.n_items + warps - 1) / warps);  // items a warp holds at a time
-  // The queue deals the items, ordered by cost, like cards: a run of cap queue positions (a warp's
-  // first items) takes every `columns`-th item, so that each warp holds items of every cost.
-  const long long columns = a.deal ? (a.n_items + cap - 1) / cap : a.n_items, rows = a.n_items / columns,
-                  longer = a.n_items % columns;  // the first `longer` columns hold one item more
-  auto dealt = [&](long long pos) {
-    const long long head = longer * (rows + 1);
-    const long long w = pos < head ? pos / (rows + 1) : longer + (pos - head) / rows;
-    const long long j = pos < head ? pos % (rows + 1) : (pos - head) % rows;
-    return j * columns + w;
-  };
+  const int cap = (int)min((long long)EDGE_CAP, (a.n_items + EDGE_SPLIT * warps - 1) / (EDGE_SPLIT * warps));
   bool drained = false, dirty = true;
   long long g = -1;
   unsigned long long my_attempts = 0, my_accepted = 0, my_spec = 0, my_discarded = 0;
@@ -537,43 +528,43 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
       __syncwarp();
     }
   };
+  // Items for idle lanes, at most `most`, from the queue.
+  auto take_items = [&](int most) {
+    const unsigned idle = __ballot_sync(FULL, role == EDGE_IDLE);
+    const int want = min(__popc(idle), most);
+    if (drained || want <= 0) return;
+    unsigned long long base = 0;
+    const int leader = __ffs(idle) - 1;
+    if ((int)lane == leader) base = atomicAdd(&a.q->head, (unsigned long long)want);
+    base = __shfl_sync(FULL, base, leader);
+    if (base + (unsigned long long)want >= (unsigned long long)a.n_items) drained = true;
+    const int rank = __popc(idle & lt_mask);
+    if (role == EDGE_IDLE && rank < want) {
+      const unsigned long long mine = base + (unsigned long long)rank;
+      if (mine < (unsigned long long)a.n_items) {
+        g = a.order[mine];
+        L.c = a.item_case[g];
+        L.lo = a.lo[g];
+        L.hi = a.hi[g];
+        L.cphi = a.cos_phi[g];
+        L.sphi = a.sin_phi[g];
+        L.star = a.star[g];
+        L.fails = 0;
+        L.it = 0;
+        role = EDGE_OWNER;
+        if (a.iterations > 0) edge_start<M>(a, L);
+        else finish_item();
+      }
+    }
+    __syncwarp();
+  };
   while (true) {
     resolve();
-    // New items from the queue for idle lanes.
-    const unsigned idle = __ballot_sync(FULL, role == EDGE_IDLE);
-    const int n_idle = __popc(idle);
-    const int want_items = min(n_idle, cap - __popc(__ballot_sync(FULL, role == EDGE_OWNER)));
-    if (!drained && want_items > 0 && (n_idle >= a.refill_threshold || n_idle == 32)) {
-      dirty = true;
-      unsigned long long base = 0;
-      const int leader = __ffs(idle) - 1;
-      if ((int)lane == leader) base = atomicAdd(&a.q->head, (unsigned long long)want_items);
-      base = __shfl_sync(FULL, base, leader);
-      if (base + (unsigned long long)want_items >= (unsigned long long)a.n_items) drained = true;
-      const int rank = __popc(idle & lt_mask);
-      if (role == EDGE_IDLE && rank < want_items) {
-        const unsigned long long mine = base + (unsigned long long)rank;
-        if (mine < (unsigned long long)a.n_items) {
-          g = a.order[dealt((long long)mine)];
-          L.c = a.item_case[g];
-          L.lo = a.lo[g];
-          L.hi = a.hi[g];
-          L.cphi = a.cos_phi[g];
-          L.sphi = a.sin_phi[g];
-          L.star = a.star[g];
-          L.fails = 0;
-          L.it = 0;
-          role = EDGE_OWNER;
-          if (a.iterations > 0) edge_start<M>(a, L);
-          else finish_item();
-        }
-      }
-      resolve();
-    }
-    // With no more items to take: idle lanes take the untraced nodes below the owners' brackets,
-    // along the predicted paths first, shallowest first, then in lane order of the owners.
-    if (dirty && (drained || __popc(__ballot_sync(FULL, role == EDGE_OWNER)) >= cap)) {
+    // Idle lanes: up to `cap` items, then the nodes along the owners' predicted paths, then further
+    // items, and once the queue is drained the nodes of the trees below the paths' ends.
+    if (dirty) {
       dirty = false;
+      take_items(cap - __popc(__ballot_sync(FULL, role == EDGE_OWNER)));
       const unsigned idle2 = __ballot_sync(FULL, role == EDGE_IDLE);
       const int n_idle2 = __popc(idle2);
       if (idle2) {
@@ -625,10 +616,12 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
           }
           base_rank += __popc(open);
         }
-        // The tree below the paths' ends.  The owners with the most work left (halvings left x
-        // rtol^-1/5, the DP5 step count's growth) come first: those at least half the warp's
-        // largest, then the others.
+        // The tree below the paths' ends, for the lanes that neither a path nor an item takes.  The
+        // owners with the most work left (halvings left x rtol^-1/5, the DP5 step count's growth)
+        // come first: those at least half the warp's largest, then the others.
         const bool in_chain = h >= 0;
+        const bool more = !drained;  // items before trees
+
         float work = 0.0f;
         if (role == EDGE_OWNER)
           work = (float)(a.iterations - L.it) * exp2f(-0.2f * __log2f((float)params(L.c).rtol));
@@ -636,7 +629,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(FULL, wmax, off));
         const bool heavy = work >= 0.5f * wmax;
-        for (int pd = 0; pd < 2 * EDGE_DEPTH && base_rank < n_idle2; ++pd) {
+        for (int pd = 0; pd < 2 * EDGE_DEPTH && base_rank < n_idle2 && !more; ++pd) {
           const int t = pd % EDGE_DEPTH + 1;
           const bool this_pass = (pd < EDGE_DEPTH) == heavy;
           const int width = 1 << t;
@@ -703,7 +696,14 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
           edge_start<M>(a, L);
         }
         __syncwarp();
+        if (more) {
+          take_items(32);
+        }
+        // trees for what the queue left idle, or the next items (none to trace: iterations = 0)
+        if (more && __ballot_sync(FULL, role == EDGE_IDLE)) dirty = true;
       }
+      resolve();
+      if (dirty) continue;
     }
     const unsigned busy = __ballot_sync(FULL, role != EDGE_IDLE && L.ry.state == RUNNING);
     if (busy == 0) {
@@ -744,19 +744,8 @@ cudaError_t run_bisect_as(EdgeArgs a, cudaStream_t s) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // Blocks per SM: the most, up to what fits, whose lanes number at most 3/4 of the items, so
-  // that lanes which finish take further items from the queue; a study smaller than that keeps
-  // every resident block, its idle lanes tracing midpoints ahead.  (The 51,840-item edge study
-  // ran 131 ms at 2 blocks per SM, 147 ms at 3 and 181 ms at 1; every bracket the same.)
-  int bps = nb;
-  for (int b = nb; b >= 1; --b) {
-    if (4LL * sms * b * MAXT <= 3LL * a.n_items) {
-      bps = b;
-      break;
-    }
-  }
   a.block = MAXT;
-  a.grid = sms * bps;
+  a.grid = sms * nb;
   k_bisect_edges<M, MAXT, MINB, SMEM><<<a.grid, MAXT, smem, s>>>(a);
   return cudaGetLastError();
 }

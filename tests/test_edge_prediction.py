@@ -1,4 +1,4 @@
-"""The edge bisection's predicted path and dealt queue: whatever the prediction, the brackets and
+"""The edge bisection's predicted path and spread queue: whatever the prediction, the brackets and
 lost-photon counts are the sequential bisection's, bit for bit."""
 
 from __future__ import annotations
@@ -44,9 +44,9 @@ def test_short_and_long_chains(rtol, iterations):
     _check([_case(0.7, 40.0, 1.0e3, rtol, 3, 2.0, 8.0)], iterations, "fast64")
 
 
-@pytest.mark.parametrize("n", [1, 2, 1183, 1185, 2369, 5000])
-def test_items_around_multiples_of_the_warps(n):
-    """1184 warps at two blocks per SM: runs of one, two and more items, the last rows ragged."""
+@pytest.mark.parametrize("n", [1, 2, 1183, 1185, 4736, 4737, 9000])
+def test_items_around_the_warps_shares(n):
+    """1184 warps at two blocks per SM, 1776 at three: a share of one item, of more, and the other build (above 4736)."""
     half = n // 2
     cases = [_case(0.9, 60.0, 1.0e3, 1e-5, n - half, 2.0, 8.0)]
     if half:
