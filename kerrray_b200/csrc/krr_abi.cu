@@ -518,6 +518,21 @@ int persistent_shape(int device, int32_t precision, const krr_options* o, const 
   return KRR_OK;
 }
 
+// Whether a host batch is traced long photons first (krr::trace_order): rows of unknown order, or
+// several images of one tolerance (of several, the caller's order of images tells more), with more
+// photons than resident lanes of variant 0 (fewer all start at once) and at most 32 times as many
+// (beyond, the tail it shortens is small: 1M random rays 4-7 % of the trace).
+bool order_wanted(int device, int32_t precision, const krr_image* images, int n_images, bool rows, long long total) {
+  if (!rows && n_images < 2) return false;
+  for (int k = 1; k < n_images; ++k)
+    if (images[k].options.rtol != images[0].options.rtol) return false;
+  int count = 0;
+  const krr::Variant* vs = variants_for(precision, &images[0].options, &count);
+  if (!vs || count < 1) return false;
+  const long long lanes = (long long)sm_count_of(device) * std::max(vs[0].occupancy(), 0) * vs[0].block;
+  return total > lanes && total <= 32 * lanes;
+}
+
 // Device layout of a batched launch's workspace: four queue counters (the main trace; the
 // reference-order trace of the edge or of the critical photons; with the critical set, the
 // FP64 re-trace of photons unlike their analytic class and the reference-order re-trace of
@@ -545,6 +560,10 @@ size_t work_bytes(int n_images, long long list_entries) {
   const size_t n = (size_t)std::max(list_entries, 0LL);
   return kQueueArea + round256((size_t)std::max(n_images, 0) * sizeof(krr::Image)) + 2 * round256(n * 8) + n;
 }
+
+// A workspace with room for the trace order (8 bytes per photon) behind the rest.
+size_t order_at(int n_images) { return round256(work_bytes(n_images, 0)); }
+size_t work_bytes_ordered(int n_images, long long total) { return order_at(n_images) + round256((size_t)total * 8); }
 
 WorkLayout work_layout(void* base, int n_images, long long list_entries) {
   char* b = static_cast<char*>(base);
@@ -574,6 +593,7 @@ struct Pipeline {
   bool dtype32 = false, rk4 = false, disk = false;
   bool retrace = false;
   int retrace_mode = 0;  // KRR_RETRACE_*
+  long long* order = nullptr;  // the trace order, made before the main trace (null: the queue's own)
   WorkLayout w{};
   krr_result out{};
   krr::PersistArgs main{};
@@ -787,9 +807,20 @@ cudaError_t enqueue_pipeline(const Pipeline& p, cudaStream_t s, cudaEvent_t ev0,
   if (e == cudaSuccess && p.out.event_Y) e = cudaMemsetAsync(p.out.event_Y, 0, (size_t)p.total * 8 * sizeof(double), s);
   if (e == cudaSuccess && p.out.event_hit) e = cudaMemsetAsync(p.out.event_hit, 0, (size_t)p.total, s);
   if (e == cudaSuccess && ev0) e = cudaEventRecord(ev0, s);
+  if (e == cudaSuccess && p.order) {
+    krr::OrderArgs oa{};
+    oa.images = p.w.images;
+    oa.n_images = p.n_images;
+    oa.Y0 = p.main.Y0;
+    oa.total = p.total;
+    oa.order = p.order;
+    oa.q = p.w.q0;
+    e = krr::trace_order(oa, s);
+  }
   if (e != cudaSuccess) return e;
   if (p.plain) {
     krr::PlainArgs pa{};
+    pa.index = p.order;
     pa.images = p.w.images;
     pa.n_images = p.n_images;
     pa.Y0 = p.main.Y0;
@@ -861,10 +892,12 @@ int finish_pipeline(const Pipeline& p, cudaStream_t s, krr_stats* stats, cudaEve
 
 int run_images(Context* c, const krr_image* images, const std::vector<krr::Image>& ims, long long total,
                const double* d_Y0, const krr_launch* launch, const krr_result* d_out, void* d_work, size_t work_size,
-               cudaStream_t s, krr_stats* stats) {
+               cudaStream_t s, krr_stats* stats, long long* order = nullptr) {
   Pipeline p;
   int rc = prepare_pipeline(c->device, images, (int)ims.size(), total, d_Y0, launch, d_out, d_work, work_size, p);
   if (rc) return rc;
+  p.order = order;
+  p.main.index = order;
   KRR_CUDA(cudaMemcpyAsync(p.w.images, ims.data(), ims.size() * sizeof(krr::Image), cudaMemcpyHostToDevice, s));
   KRR_CUDA(enqueue_pipeline(p, s, c->ev0, c->ev1, c->ev2));
   return finish_pipeline(p, s, stats, c->ev0, c->ev1, c->ev2);
@@ -1093,26 +1126,45 @@ int krr_integrate_batch(int device, double mass, double spin, const double* Y0, 
     LaunchShape shape{};
     rc = persistent_shape(device, precision, options, nullptr, n, shape);
     if (rc) return rc;
+    krr_image im0{};
+    im0.options = *options;
+    const bool ordered = order_wanted(device, precision, &im0, 1, true, n);
+    WorkLayout w{};
+    long long* order = nullptr;
+    krr::Image im{};
+    im.P = make_params(mass, spin, options);
+    im.count = n;
+    if (ordered || shape.plain_block == 0) {
+      KRR_CUDA(c->buf[B_QUEUE].ensure(work_bytes_ordered(1, ordered ? n : 0)));
+      w = work_layout(c->buf[B_QUEUE].p, 1, 0);
+      KRR_CUDA(cudaMemsetAsync(w.q0, 0, sizeof(krr::Queue), c->stream));
+      KRR_CUDA(cudaMemcpyAsync(w.images, &im, sizeof(im), cudaMemcpyHostToDevice, c->stream));
+    }
+    if (ordered) {
+      order = reinterpret_cast<long long*>(static_cast<char*>(c->buf[B_QUEUE].p) + order_at(1));
+      krr::OrderArgs oa{};
+      oa.P = im.P;
+      oa.Y0 = d_Y0;
+      oa.total = n;
+      oa.order = order;
+      oa.q = w.q0;
+      KRR_CUDA(krr::trace_order(oa, c->stream));
+    }
     if (shape.plain_block > 0) {
       krr::PlainArgs a{};
-      a.P = make_params(mass, spin, options);
+      a.P = im.P;
       a.Y0 = d_Y0;
+      a.index = order;
       a.n = n;
       a.o = to_outputs(&dev);
       KRR_CUDA(launch_plain(precision, options, a, shape.plain_block, c->stream));
     } else {
-      krr::Image im{};
-      im.P = make_params(mass, spin, options);
-      im.count = n;
-      KRR_CUDA(c->buf[B_QUEUE].ensure(work_bytes(1, 0)));
-      const WorkLayout w = work_layout(c->buf[B_QUEUE].p, 1, 0);
-      KRR_CUDA(cudaMemsetAsync(w.q0, 0, sizeof(krr::Queue), c->stream));
-      KRR_CUDA(cudaMemcpyAsync(w.images, &im, sizeof(im), cudaMemcpyHostToDevice, c->stream));
       krr::PersistArgs a{};
       a.images = w.images;
       a.n_images = 1;
       a.total = n;
       a.Y0 = d_Y0;
+      a.index = order;
       a.o = to_outputs(&dev);
       a.q = w.q0;
       a.refill_threshold = shape.refill;
@@ -1667,11 +1719,16 @@ int krr_trace_images(int device, const krr_image* images, int32_t n_images, cons
   krr_result dev;
   rc = device_results(c, total, out, images[0].options.disk_plane != 0, &dev);
   if (rc) return rc;
-  const size_t wbytes = work_bytes(n_images, (launch && launch->retrace) ? total : 0);
+  const bool ordered = !overlapped && !(launch && (launch->retrace || launch->plain)) &&
+                       order_wanted(device, launch ? launch->precision : (int32_t)KRR_PREC_FAST64, images, n_images,
+                                    Y0 != nullptr, total);
+  const size_t wbytes = ordered ? work_bytes_ordered(n_images, total)
+                                : work_bytes(n_images, (launch && launch->retrace) ? total : 0);
   KRR_CUDA(c->buf[B_QUEUE].ensure(wbytes));
   if (overlapped)
     return run_images_overlapped(c, images, ims, total, Y0, launch, &dev, out, c->buf[B_QUEUE].p, wbytes, stats);
-  rc = run_images(c, images, ims, total, d_Y0, launch, &dev, c->buf[B_QUEUE].p, wbytes, c->stream, stats);
+  long long* order = ordered ? reinterpret_cast<long long*>(static_cast<char*>(c->buf[B_QUEUE].p) + order_at(n_images)) : nullptr;
+  rc = run_images(c, images, ims, total, d_Y0, launch, &dev, c->buf[B_QUEUE].p, wbytes, c->stream, stats, order);
   if (rc) return rc;
   return copy_rows_back(c, &dev, out, 0, total, c->stream);
 }

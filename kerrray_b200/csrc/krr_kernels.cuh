@@ -39,6 +39,8 @@ struct Queue {
   unsigned long long flagged;     // photons appended to the re-trace list
   unsigned long long t_first;     // globaltimer (ns) of the first block's start (PDL_STAMP), from ~0
   unsigned long long t_last;      // globaltimer (ns) of the last block's end (PDL_STAMP)
+  unsigned long long order_front; // long photons placed from the front of the trace order (k_trace_order)
+  unsigned long long order_back;  // short ones placed from its back
   unsigned long long restarted;   // photons an FP32 overflow ended, traced on in place (TRACE_RESTART)
   unsigned long long speculative; // edge bisection: photons traced ahead of their bracket
   unsigned long long discarded;   // edge bisection: attempts of speculative photons not needed
@@ -863,6 +865,18 @@ __global__ void k_risk_prepass(const Image* __restrict__ images, int n_images, l
                                const double* __restrict__ Y0, unsigned char* __restrict__ risk,
                                long long* __restrict__ list, Queue* q, long long* __restrict__ near_list,
                                Queue* q_near);
+
+// The trace order of a batch: photons expected to take many steps first (k_trace_order).  Without
+// images, P holds for every row of Y0.
+struct OrderArgs {
+  Params P;
+  const Image* images;
+  int n_images;
+  const double* Y0;
+  long long total;
+  long long* order;  // total entries
+  Queue* q;          // zeroed
+};
 
 // After the traces: every non-critical photon whose code is not its analytic class, and with
 // `recheck` every photon marked RISK_RECHECK, is appended to `list` and counted in q->flagged.

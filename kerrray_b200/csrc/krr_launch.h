@@ -87,6 +87,7 @@ cudaError_t flag_boundary(const Image* images, int n_images, long long total, co
 // results against the analytic classes (disagreements appended to `list`).
 cudaError_t risk_prepass(const Image* images, int n_images, long long total, const double* Y0, unsigned char* risk,
                          long long* list, Queue* q, long long* near_list, Queue* q_near, cudaStream_t s);
+cudaError_t trace_order(const OrderArgs& a, cudaStream_t s);
 // One block of 384 threads per SM in fast FP64 (its registers fill the SM): the near-edge
 // photons of the mixed pipeline, on SMs of their own beside the mixed trace.
 const Variant* near_wide_variant();
