@@ -593,6 +593,7 @@ struct Pipeline {
   bool dtype32 = false, rk4 = false, disk = false;
   bool retrace = false;
   int retrace_mode = 0;  // KRR_RETRACE_*
+  double rtol_max = 0.0;
   long long* order = nullptr;  // the trace order, made before the main trace (null: the queue's own)
   WorkLayout w{};
   krr_result out{};
@@ -628,6 +629,7 @@ int prepare_pipeline(int device, const krr_image* images, int n_images, long lon
   p.dtype32 = o0->dtype == 1;
   p.rk4 = o0->method == 1;
   p.disk = o0->disk_plane != 0;
+  for (int k = 0; k < n_images; ++k) p.rtol_max = std::max(p.rtol_max, images[k].options.rtol);
   p.plain = launch && launch->plain;
   p.plain_block = (launch && launch->block > 0 && launch->block % 32 == 0) ? launch->block : 128;
   p.retrace_mode = launch ? launch->retrace : 0;
@@ -821,6 +823,7 @@ cudaError_t enqueue_pipeline(const Pipeline& p, cudaStream_t s, cudaEvent_t ev0,
   if (p.plain) {
     krr::PlainArgs pa{};
     pa.index = p.order;
+    pa.rtol_max = p.rtol_max;
     pa.images = p.w.images;
     pa.n_images = p.n_images;
     pa.Y0 = p.main.Y0;
@@ -1092,6 +1095,7 @@ int krr_integrate_batch_device(int device, double mass, double spin, const doubl
   a.n = n;
   a.o = to_outputs(d_out);
   a.q = nullptr;
+  a.rtol_max = options->rtol;
   KRR_CUDA(launch_plain(precision, options, a, 32, static_cast<cudaStream_t>(stream)));
   return KRR_OK;
 }
@@ -1157,6 +1161,7 @@ int krr_integrate_batch(int device, double mass, double spin, const double* Y0, 
       a.index = order;
       a.n = n;
       a.o = to_outputs(&dev);
+      a.rtol_max = options->rtol;
       KRR_CUDA(launch_plain(precision, options, a, shape.plain_block, c->stream));
     } else {
       krr::PersistArgs a{};

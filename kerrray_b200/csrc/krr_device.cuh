@@ -147,6 +147,7 @@ struct Trig {
 //             whole step to the CAREFUL form, out of line (dp_stages);
 //   ROLLED    a loop (dp_stages_loop), for kernels that keep many warps on an SM;
 //   CAREFUL   any operands, each evaluation with its own way out.
+struct NoShadow {};
 enum class Stages { UNROLLED, ROLLED, CAREFUL };
 
 template <class W, Stages FORM = Stages::UNROLLED>
@@ -162,7 +163,8 @@ struct RefMode {
 
   __device__ static Trig accept_trig(double, const Trig& tr) { return tr; }
 
-  struct Shadow {};
+  using Shadow = NoShadow;
+  using Careful = RefMode<W, Stages::CAREFUL>;
 
   __device__ static void init_rhs(const Params& P, const S y[NV], S pt, S pph, Shadow&, K f[NV], Trig& tr) {
     rhs(P, y[CR], y[CTH], pt, y[CPR], y[CPTH], pph, f, tr);
@@ -383,14 +385,17 @@ __device__ __forceinline__ float rcp_fast(float x) {
 // d^6 (|d| <= 1/4: below 4e-10).  The stages of one step move theta by such small amounts, so
 // this replaces a full sincos (argument reduction and two polynomials) by about a dozen fused
 // operations.  Returns false, computing nothing, when |d| exceeds the range.
-__device__ __forceinline__ bool sincos_shift(double s0, double c0, double d, double& s, double& c) {
-  if (!(fabs(d) <= 0.1)) return false;
+__device__ __forceinline__ void sincos_shift_values(double s0, double c0, double d, double& s, double& c) {
   const double d2 = d * d;
   const double sd = d * fma(d2, fma(d2, fma(d2, fma(d2, 1.0 / 362880.0, -1.0 / 5040.0), 1.0 / 120.0), -1.0 / 6.0), 1.0);
   const double cd =
       fma(d2, fma(d2, fma(d2, fma(d2, fma(d2, -1.0 / 3628800.0, 1.0 / 40320.0), -1.0 / 720.0), 1.0 / 24.0), -0.5), 1.0);
   s = fma(s0, cd, c0 * sd);
   c = fma(c0, cd, -(s0 * sd));
+}
+__device__ __forceinline__ bool sincos_shift(double s0, double c0, double d, double& s, double& c) {
+  if (!(fabs(d) <= 0.1)) return false;
+  sincos_shift_values(s0, c0, d, s, c);
   return true;
 }
 
@@ -567,7 +572,21 @@ struct Fast64 {
 #pragma unroll
     for (int i = 0; i < NV; ++i) ys[i] = upd<Fast64>(ry.y[i], h, acc[i]);
     double s, c;
-    if constexpr (LAST) {
+    if constexpr (R::Mode::kStraight) {
+      if constexpr (LAST) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) yn[i] = ys[i];
+        const bool near = fabs(ys[CTH]) < 1000.0;
+        const double x = near ? ys[CTH] : 0.0;
+        __builtin_assume(fabs(x) < 1000.0);
+        sincos(x, &s, &c);
+        tr.ok = tr.ok && near;
+      } else {
+        const double d = ys[CTH] - ry.y[CTH];
+        sincos_shift_values(ry.tr.s, ry.tr.c, d, s, c);
+        tr.ok = tr.ok && fabs(d) <= 0.1;
+      }
+    } else if constexpr (LAST) {
 #pragma unroll
       for (int i = 0; i < NV; ++i) yn[i] = ys[i];
       sincos(ys[CTH], &s, &c);
@@ -595,6 +614,15 @@ struct Fast64 {
     mo.set(pt, pph, P.a);
     rhs_separated<double>(fma(r, r - P.two_m, P.a2), r, s, c, pr, pth, mo, P.a, P.a2, P.mass, f);
   }
+};
+
+// Fast64 without a branch between the stages (as RefMode's UNROLLED form): every inner stage's sine
+// and cosine by the small-angle shift, and a step that turns theta by more than 0.1 done over by
+// Fast64, out of line.  For tight tolerances, whose steps are short: of the accepted steps of a
+// +-8 M image 9 % turn further at rtol 1e-6, 0.3 to 1 % at 1e-8, none at 1e-10.
+struct Fast64Straight : Fast64 {
+  using Careful = Fast64;
+  static constexpr bool kStraight = true;
 };
 
 // FP32 stages from an FP32 shadow of the FP64 state; FP64 state accumulation, error norm,
@@ -735,6 +763,7 @@ struct MixedQueue : Mixed {
 // ------------------------------------------------------------------------------------------
 template <class M>
 struct Ray {
+  using Mode = M;
   using S = typename M::S;
   using K = typename M::K;
   S y[NV];   // t, r, theta, phi, p_r, p_theta
@@ -1175,6 +1204,8 @@ template <class M>
 struct StepStart {
   typename M::S y[NV], pt, pph;
   typename M::K f[NV], h;
+  typename M::Careful::Shadow sh;
+  Trig tr;
 };
 template <class M>
 struct StepEnd {
@@ -1184,8 +1215,10 @@ struct StepEnd {
 };
 template <class M, bool RK4>
 static __device__ __noinline__ StepEnd<M> dp_stages_careful(const Params& P, StepStart<M> a) {
-  using C = RefMode<typename M::S, Stages::CAREFUL>;
+  using C = typename M::Careful;
   Ray<C> ry;
+  ry.sh = a.sh;
+  ry.tr = a.tr;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     ry.y[i] = a.y[i];
@@ -1194,7 +1227,7 @@ static __device__ __noinline__ StepEnd<M> dp_stages_careful(const Params& P, Ste
   ry.pt = a.pt;
   ry.pph = a.pph;
   StepEnd<M> e;
-  if constexpr (RK4) dp_stages_scalar<C, true>(P, ry, a.h, e.k6, e.yn, e.esum, e.tr);
+  if constexpr (RK4 || M::kFused) dp_stages_scalar<C, RK4>(P, ry, a.h, e.k6, e.yn, e.esum, e.tr);
   else dp_stages_loop<C>(P, ry, a.h, e.k6, e.yn, e.esum, e.tr);
   return e;
 }
@@ -1221,6 +1254,8 @@ __device__ __forceinline__ void dp_stages(const Params& P, const Ray<M>& ry, typ
       a.pt = ry.pt;
       a.pph = ry.pph;
       a.h = h;
+      a.sh = ry.sh;
+      a.tr = ry.tr;
       const StepEnd<M> e = dp_stages_careful<M, RK4>(P, a);
 #pragma unroll
       for (int i = 0; i < NV; ++i) {

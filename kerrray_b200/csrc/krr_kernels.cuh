@@ -783,7 +783,11 @@ struct PlainArgs {
   long long n;
   Outputs o;
   Queue* q;
+  double rtol_max;  // the coarsest tolerance among the rays' parameters
 };
+
+// The coarsest tolerance that the fast64 stages without branches are used for (Fast64Straight).
+constexpr double kStraightRtol = 2e-9;
 
 struct PersistArgs {
   const Image* images;
