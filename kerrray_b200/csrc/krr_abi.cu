@@ -518,6 +518,12 @@ int persistent_shape(int device, int32_t precision, const krr_options* o, const 
   return KRR_OK;
 }
 
+// Four lanes per ray in reference order (krr_quad.cuh): up to two warps of eight rays per scheduler.
+bool quad_fits(int device, int32_t precision, const krr_options* o, bool events, long long n) {
+  return precision == KRR_PREC_REFERENCE && o->dtype == 0 && o->method == 0 && !events &&
+         n <= (long long)sm_count_of(device) * 4 * 16;
+}
+
 // Whether a host batch is traced long photons first (krr::trace_order): rows of unknown order, or
 // several images of one tolerance (of several, the caller's order of images tells more), with more
 // photons than resident lanes of variant 0 (fewer all start at once) and at most 32 times as many
@@ -594,6 +600,7 @@ struct Pipeline {
   bool retrace = false;
   int retrace_mode = 0;  // KRR_RETRACE_*
   double rtol_max = 0.0;
+  bool quad = false;  // plain, four lanes per ray
   long long* order = nullptr;  // the trace order, made before the main trace (null: the queue's own)
   WorkLayout w{};
   krr_result out{};
@@ -662,6 +669,9 @@ int prepare_pipeline(int device, const krr_image* images, int n_images, long lon
   if (shape.plain_block > 0 && !p.retrace && !p.plain) {
     p.plain = true;
     p.plain_block = shape.plain_block;
+    bool events = false;
+    for (int k = 0; k < n_images; ++k) events = events || images[k].options.disk_plane;
+    p.quad = quad_fits(device, precision, o0, events, total);
   }
   p.main_v = shape.v;
   p.main.images = p.w.images;
@@ -824,6 +834,7 @@ cudaError_t enqueue_pipeline(const Pipeline& p, cudaStream_t s, cudaEvent_t ev0,
     krr::PlainArgs pa{};
     pa.index = p.order;
     pa.rtol_max = p.rtol_max;
+    pa.quad = p.quad;
     pa.images = p.w.images;
     pa.n_images = p.n_images;
     pa.Y0 = p.main.Y0;
@@ -1096,6 +1107,7 @@ int krr_integrate_batch_device(int device, double mass, double spin, const doubl
   a.o = to_outputs(d_out);
   a.q = nullptr;
   a.rtol_max = options->rtol;
+  a.quad = quad_fits(device, precision, options, options->disk_plane != 0, n);
   KRR_CUDA(launch_plain(precision, options, a, 32, static_cast<cudaStream_t>(stream)));
   return KRR_OK;
 }
@@ -1162,6 +1174,7 @@ int krr_integrate_batch(int device, double mass, double spin, const double* Y0, 
       a.n = n;
       a.o = to_outputs(&dev);
       a.rtol_max = options->rtol;
+      a.quad = quad_fits(device, precision, options, options->disk_plane != 0, n);
       KRR_CUDA(launch_plain(precision, options, a, shape.plain_block, c->stream));
     } else {
       krr::PersistArgs a{};

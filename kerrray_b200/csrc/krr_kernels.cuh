@@ -784,6 +784,7 @@ struct PlainArgs {
   Outputs o;
   Queue* q;
   double rtol_max;  // the coarsest tolerance among the rays' parameters
+  bool quad;        // four lanes per ray (k_trace_quad: reference order, rk45, float64, no disk event)
 };
 
 // The coarsest tolerance that the fast64 stages without branches are used for (Fast64Straight).

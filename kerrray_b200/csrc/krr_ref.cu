@@ -4,10 +4,14 @@
 #include <math_constants.h>
 
 #include "krr_launch.h"
+#include "krr_quad.cuh"
 
 namespace krr {
 
+static cudaError_t ref_quad(const PlainArgs& a, cudaStream_t s);
+
 cudaError_t ref_plain(bool dtype32, bool rk4, const PlainArgs& a, int block, cudaStream_t s) {
+  if (a.quad) return ref_quad(a, s);
   if (dtype32) return rk4 ? run_plain<RefMode<float>, true>(a, block, s) : run_plain<RefMode<float>, false>(a, block, s);
   return rk4 ? run_plain<RefMode<double>, true>(a, block, s) : run_plain<RefMode<double>, false>(a, block, s);
 }
@@ -30,6 +34,53 @@ const Variant* ref_variants(bool dtype32, bool rk4, int* count) {
 }
 
 cudaError_t ref_bisect(const EdgeArgs& a, cudaStream_t s) { return run_bisect<RefMode<double>, 128, 1>(a, s); }
+
+__global__ void __launch_bounds__(128) k_trace_quad(const __grid_constant__ Params P, const Image* __restrict__ images,
+                                                    int n_images, const double* __restrict__ Y0,
+                                                    const long long* __restrict__ index, long long n, Outputs o, Queue* q) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const long long i = (blockIdx.x * 128LL + threadIdx.x) >> 2;
+  const bool mine = i < n;
+  const long long g = mine ? (index ? index[i] : i) : (index ? index[0] : 0);  // lanes without a ray idle on the first
+  const int img = images ? find_image(images, n_images, g) : 0;
+  const Params& Pi = images ? images[img].P : P;
+  double y0[8];
+  photon_source(images, img, Y0, g, y0, mine ? q : nullptr);
+  Quad ray;
+  ray.start(Pi, y0, carter_initial(Pi, y0));
+  if (!mine) ray.state = FAILURE;
+  unsigned iters = 0;
+  while (__any_sync(FULL, ray.state == RUNNING)) {
+    ray.attempt(Pi, ray.state == RUNNING);
+    __syncwarp();
+    iters += 1;
+  }
+  if (mine) ray.store(o, g);
+  if (q) {
+    const bool counts = mine && (threadIdx.x & 3u) == 0;
+    unsigned long long n_att = counts ? (unsigned long long)ray.attempts : 0, n_acc = counts ? (unsigned long long)ray.n_steps : 0;
+    unsigned long long n_ret = counts ? 1 : 0;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      n_att += __shfl_down_sync(FULL, n_att, off);
+      n_acc += __shfl_down_sync(FULL, n_acc, off);
+      n_ret += __shfl_down_sync(FULL, n_ret, off);
+    }
+    if ((threadIdx.x & 31u) == 0 && n_ret) {
+      atomicAdd(&q->retired, n_ret);
+      atomicAdd(&q->attempts, n_att);
+      atomicAdd(&q->accepted, n_acc);
+      atomicAdd(&q->lane_iters, (unsigned long long)iters * 32ull);
+      atomicAdd(&q->busy_iters, n_att);
+    }
+  }
+}
+
+static cudaError_t ref_quad(const PlainArgs& a, cudaStream_t s) {
+  if (a.n <= 0) return cudaSuccess;
+  k_trace_quad<<<(unsigned)((4 * a.n + 127) / 128), 128, 0, s>>>(a.P, a.images, a.n_images, a.Y0, a.index, a.n, a.o, a.q);
+  return cudaGetLastError();
+}
 
 // Eight warps per block: at the reference order's register count one block fills an SM's
 // register file, so the critical photons of the mixed pipeline hold SMs of their own.
