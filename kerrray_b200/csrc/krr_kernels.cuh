@@ -350,15 +350,19 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // to the first photon closer than that (its length is the owner's `chain`: about 20 levels of a
 // 6 M bracket at rtol 1e-6, 31 at 1e-10), are traced first; lanes that no path needs take further
 // items, most expensive first; and once the queue is drained, the tree below the paths' ends, where
-// either outcome is possible.  A wrong prediction costs the attempts of the nodes below it, nothing
-// else.
+// either outcome is possible.  From then on a photon's radial momentum tells its outcome too, about
+// halfway along its steps (edge_shows): the edge then lies between the outermost photon that falls in
+// and the innermost that gets out, and lanes of brackets beside those two start on the levels below
+// while the photons above are still running, so that the levels overlap.  A wrong prediction costs the
+// attempts of the nodes below it, nothing else.
 //
 // Measured (kernel, B200).  One edge, 90 directions, 36 halvings, rtol 1e-6, reference order: 87 ms
-// with the first three warps holding every item, 20 ms now (2000 attempts per warp for 36 halvings
-// of 341 each).  12 cases x 241 directions x 3 tolerances, fast64: 110 -> 31 ms; with an even share of
-// the items per warp from the start (8 a warp, dealt so that each holds every tolerance) 36 ms.
-// x 1440 directions (51,840 items): 127 -> 100 ms, 115 with an even share.  EDGE_CONF 2 and 16 within
-// 5 % of 4 on all three.
+// with the first three warps holding every item, 20 ms with the paths and trees (2000 attempts per
+// warp for 36 halvings of 341 each), 12.8-14 ms with the outcomes told ahead (1290 attempts; at rtol
+// 1e-8 31-34 -> 21-25 ms).  12 cases x 241 directions x 3 tolerances, fast64: 110 -> 32-35 -> 28-31 ms;
+// with an even share of the items per warp from the start (8 a warp, dealt so that each holds every
+// tolerance) 36 ms.  x 1440 directions (51,840 items): 127 -> 100 ms, 115 with an even share.
+// EDGE_CONF 1 to 16 and EDGE_OFF 1 and 3 within 5 %; so is waiting until 4 to 12 lanes are free.
 // ------------------------------------------------------------------------------------------
 struct EdgeCase {
   Params P;
@@ -389,7 +393,9 @@ struct EdgeLane {
   double lo, hi, mid, cphi, sphi, star;
   long long fails;
   int it, c;
+  float inward;  // -Delta p_r after the photon's last step; EDGE_OUT or EDGE_IN once it shows the outcome
 };
+constexpr float EDGE_OUT = -1.0f, EDGE_IN = -2.0f;
 
 template <class M>
 __device__ __forceinline__ void edge_start(const EdgeArgs& a, EdgeLane<M>& L) {
@@ -400,6 +406,24 @@ __device__ __forceinline__ void edge_start(const EdgeArgs& a, EdgeLane<M>& L) {
   double y0[8];
   if (camera_state(ec.F, al, be, y0) != 0) atomicCAS(&a.q->error, 0, 6);
   ray_init<M>(ec.P, y0, carter_initial(ec.P, y0), L.ry);
+  L.inward = INFINITY;
+}
+
+// Where a running photon will end, as far as its radial momentum shows: (Delta p_r)^2 = R(r), and R
+// falls inwards to its minimum beside the photon orbits.  A photon that moves outwards has met its
+// turning point; one that moves inwards past the minimum has none left.  A photon near the edge shows
+// this about halfway along its steps.  The outcome itself is what the finished photon gives: this
+// only chooses what is traced ahead.  Whether it shows it with this step:
+template <class M>
+__device__ __forceinline__ bool edge_shows(const Params& P, EdgeLane<M>& L) {
+  if (L.ry.state != RUNNING) return true;
+  if (L.inward < 0.0f) return false;
+  const double r = (double)L.ry.y[CR];
+  const float w = (float)-(fma(r, r - P.two_m, P.a2) * (double)L.ry.y[CPR]);
+  if (w < 0.0f) L.inward = EDGE_OUT;
+  else if (w > L.inward) L.inward = EDGE_IN;
+  else L.inward = w;
+  return L.inward < 0.0f;
 }
 
 enum : int { EDGE_IDLE = 0, EDGE_OWNER = 1, EDGE_HELPER = 2 };
@@ -456,6 +480,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
   L.lo = L.hi = L.mid = L.cphi = L.sphi = L.star = 0.0;
   L.fails = 0;
   L.it = L.c = 0;
+  L.inward = INFINITY;
   int role = EDGE_IDLE, host = 0, depth = 0;
   unsigned path = 0;
   const long long warps = (long long)gridDim.x * (MAXT / 32);
@@ -567,26 +592,66 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
     if (dirty) {
       dirty = false;
       take_items(cap - __popc(__ballot_sync(FULL, role == EDGE_OWNER)));
+      // With no item left to take: the outcomes that each owner's photons show bound its edge to
+      // (in_m, out_m), and photons of brackets outside it give up their lanes.
+      double in_m = -INFINITY, out_m = INFINITY;
+      if (drained) {
+        int shown = -1;
+        if (role != EDGE_IDLE) {
+          if (L.ry.state != RUNNING) shown = L.ry.state == ESCAPED ? 1 : 0;
+          else if (L.inward < 0.0f) shown = L.inward == EDGE_OUT ? 1 : 0;
+        }
+        const int code = 2 * (role == EDGE_HELPER ? host : (int)lane) + shown;
+        for (unsigned todo = __ballot_sync(FULL, shown >= 0); todo; todo &= todo - 1u) {
+          const int k = __ffs(todo) - 1;
+          const double m = __shfl_sync(FULL, L.mid, k);
+          const int ck = __shfl_sync(FULL, code, k);
+          if ((ck >> 1) == (int)lane) {
+            if (ck & 1) out_m = fmin(out_m, m);
+            else in_m = fmax(in_m, m);
+          }
+        }
+        const int hl = (role == EDGE_HELPER) ? host : (int)lane;
+        const double host_in = __shfl_sync(FULL, in_m, hl), host_out = __shfl_sync(FULL, out_m, hl);
+        if (role == EDGE_HELPER && L.lo < L.hi && (L.hi <= host_in || L.lo >= host_out)) {
+          my_discarded += (unsigned long long)L.ry.attempts;
+          role = EDGE_IDLE;
+        }
+      }
       const unsigned idle2 = __ballot_sync(FULL, role == EDGE_IDLE);
       const int n_idle2 = __popc(idle2);
       if (idle2) {
         // The owners' predicted paths.
         int chain = 0;
-        unsigned cpath = 0;
+        unsigned cpath = 0, dead = 0;
         const int below = (role == EDGE_OWNER) ? a.iterations - 1 - L.it : 0;  // levels below the owner's photon
         if (below > 0) {
           const Params& Pc = params(L.c);
           // a bracket that no longer holds `star` shows how far off it is at least
-          const double off = fmax(fmax(L.lo - L.star, L.star - L.hi), 0.0);
+          const double off = fmax(fmax(fmax(L.lo, in_m) - L.star, L.star - fmin(L.hi, out_m)), 0.0);
           const double conf = EDGE_CONF * Pc.rtol * Pc.mass + EDGE_OFF * off;
           const int most = min(below, EDGE_CHAIN);
           double lo_c = L.lo, hi_c = L.hi, mid = L.mid;
-          while (chain < most && fabs(mid - L.star) > conf) {
-            const bool out = mid > L.star;
+          while (chain < most) {
+            const bool shows_in = mid <= in_m, shows_out = mid >= out_m;
+            if (!(shows_in || shows_out || fabs(mid - L.star) > conf)) break;
+            const bool out = !shows_in && (shows_out || mid > L.star);
             cpath = 2u * cpath + (out ? 1u : 0u);
             if (out) hi_c = mid; else lo_c = mid;
             chain += 1;
             mid = 0.5 * (lo_c + hi_c);
+          }
+          // nodes of the tree below the path's end whose brackets hold no edge any more
+          if (lo_c < hi_c && (in_m > lo_c || out_m < hi_c)) {
+            double w = hi_c - lo_c;
+            for (int t = 1; t <= EDGE_DEPTH; ++t) {
+              w *= 0.5;
+              const int last = (1 << t) - 1;
+              for (int k = 0; k <= last; ++k) {
+                const double at = fma((double)k, w, lo_c);
+                if (at + w <= in_m || at >= out_m) dead |= 1u << edge_node(t, (unsigned)(last - k));
+              }
+            }
           }
         }
         slot[lane] = slot2[lane] = 0;
@@ -604,7 +669,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
           }
         }
         __syncwarp();
-        const unsigned on_chain = (unsigned)slot[lane], in_tree = (unsigned)slot2[lane];
+        const unsigned on_chain = (unsigned)slot[lane], in_tree = (unsigned)slot2[lane] | dead;
         const int rank = (role == EDGE_IDLE) ? __popc(idle2 & lt_mask) : -1;
         int h = -1, hd = 0, base_rank = 0;  // the node taken: owner lane, depth, path
         unsigned hp = 0;
@@ -713,10 +778,13 @@ __global__ void __launch_bounds__(MAXT, MINB) k_bisect_edges(EdgeArgs a) {
       continue;
     }
     my_iters += 1;
+    bool shows = false;
     if (role != EDGE_IDLE && L.ry.state == RUNNING) {
       attempt<M, false>(params(L.c), L.ry, nullptr, nullptr);
       my_attempts += 1;
+      if (drained) shows = edge_shows<M>(params(L.c), L);
     }
+    if (drained && __any_sync(FULL, shows)) dirty = true;
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {

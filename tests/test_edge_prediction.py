@@ -52,3 +52,12 @@ def test_items_around_the_warps_shares(n):
     if half:
         cases.append(_case(0.5, 17.0, 1.0e3, 1e-6, half, 2.0, 8.0))
     _check(cases, 6, "fast64")
+
+
+@pytest.mark.parametrize("r_o,lo,hi", [(1.0e3, 2.0, 8.0), (6.0, 0.5, 4.0), (3.0, 0.1, 1.4), (1.0e3, 0.0, 200.0)])
+@pytest.mark.parametrize("n", [1, 33, 180])
+def test_outcomes_told_ahead(r_o, lo, hi, n):
+    """Few items, so that lanes start below photons that still run: from far, from beside the photon orbits
+    and inside them (where the radial momentum tells little or the wrong side), and in a wide bracket."""
+    for precision, rtol in (("reference", 1e-6), ("fast64", 1e-10), ("mixed", 1e-6)):
+        _check([_case(0.9, 60.0, r_o, rtol, n, lo, hi)], 36, precision)
