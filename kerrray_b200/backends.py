@@ -55,10 +55,12 @@ class Backend(Protocol):
 
 
 def _validate_batch(Y0: ArrayLike) -> np.ndarray:
-    arr = np.asarray(Y0, dtype=np.float64)
+    # A private copy: the library reads the rows after the GIL is released, so a caller's thread that
+    # writes to its array must not reach rows that were, or are about to be, checked.
+    arr = np.array(Y0, dtype=np.float64, order="C")
     if arr.ndim != 2 or arr.shape[1] != STATE_SIZE:
         raise ValueError(f"Y0 must have shape (N, {STATE_SIZE}), got {arr.shape}")
-    return np.ascontiguousarray(arr)  # the library checks that every value is finite
+    return arr  # the library checks that every value is finite
 
 
 def _result_type():
