@@ -5,7 +5,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <thread>
 #include <chrono>
 #include <climits>
 #include <cmath>
@@ -18,6 +17,7 @@
 #include <vector>
 
 #include "../../include/kerrray_cuda.h"
+#include "krr_finite.h"
 #include "krr_host.h"
 #include "krr_launch.h"
 #include "krr_staging.h"
@@ -252,32 +252,6 @@ int get_context(int device, Context** out) {
   }
   *out = g_ctx[device].get();
   return KRR_OK;
-}
-
-// Every value finite: a branch-free pass over the exponent fields (vectorised by the host
-// compiler; an early-exit isfinite loop ran at a fraction of the memory bandwidth).
-bool all_finite(const double* x, size_t n) {
-  const uint64_t* b = reinterpret_cast<const uint64_t*>(x);
-  constexpr uint64_t kExp = 0x7ff0000000000000ull;
-  uint64_t bad = 0;
-  for (size_t i = 0; i < n; ++i) bad |= (uint64_t)((b[i] & kExp) == kExp);
-  return bad == 0;
-}
-
-// all_finite over up to 16 host threads for large arrays (memory-bandwidth bound).
-bool all_finite_parallel(const double* x, size_t n) {
-  const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  if (n < ((size_t)1 << 22) || hw == 1) return all_finite(x, n);
-  std::vector<char> ok(hw, 1);
-  std::vector<std::thread> threads;
-  const size_t per = (n + hw - 1) / hw;
-  for (unsigned t = 0; t < hw; ++t)
-    threads.emplace_back([&, t] {
-      const size_t a = t * per, b = std::min(n, a + per);
-      if (a < b) ok[t] = all_finite(x + a, b - a);
-    });
-  for (auto& th : threads) th.join();
-  return std::all_of(ok.begin(), ok.end(), [](char v) { return v != 0; });
 }
 
 // Host doubles to the device on stream s, through the staging memory if they are pageable; *bad
