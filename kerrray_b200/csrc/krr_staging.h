@@ -40,7 +40,8 @@ struct CopySpan {
 };
 
 // Owned by a device context and used under its lock: at most kSlots x kSlotBytes of pinned memory,
-// allocated in groups as transfers first need them and kept for the next ones.
+// allocated in groups as transfers first need them and kept for the next ones.  Where pinned memory
+// cannot be had, the transfers use the slots there are, and without any the driver's pageable copies.
 class Staging {
  public:
   static constexpr size_t kSlotBytes = (size_t)1 << 20;
@@ -63,26 +64,35 @@ class Staging {
   cudaEvent_t ev_[kSlots] = {};
   int have_ = 0;
 
-  cudaError_t ensure(int n) {
+  // Slots for n pieces, or as many as there is pinned memory for (perhaps none).
+  void ensure(int n) {
     while (have_ < std::min(n, kSlots)) {
       char* p = nullptr;
-      cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&p), kGroup * kSlotBytes, cudaHostAllocDefault);
-      if (e != cudaSuccess) {
-        if (have_ == 0) return e;
-        cudaGetLastError();  // go on with the slots there are
-        return cudaSuccess;
+      if (cudaHostAlloc(reinterpret_cast<void**>(&p), kGroup * kSlotBytes, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return;
       }
       for (int k = 0; k < kGroup; ++k) {
-        if ((e = cudaEventCreateWithFlags(&ev_[have_ + k], cudaEventDisableTiming)) != cudaSuccess) {
+        if (cudaEventCreateWithFlags(&ev_[have_ + k], cudaEventDisableTiming) != cudaSuccess) {
+          cudaGetLastError();
           for (int j = 0; j < k; ++j) cudaEventDestroy(ev_[have_ + j]);
           cudaFreeHost(p);
-          return e;
+          return;
         }
         slot_[have_ + k] = p + (size_t)k * kSlotBytes;
       }
       have_ += kGroup;
     }
-    return cudaSuccess;
+  }
+
+  // Without any slot: the driver's own copies of pageable memory.
+  static cudaError_t copy_plain(const std::vector<CopySpan>& spans, cudaStream_t s, bool out, std::atomic<bool>* bad) {
+    for (const CopySpan& x : spans) {
+      if (bad && !finite_doubles(static_cast<const char*>(x.src), x.bytes)) bad->store(true);
+      const cudaError_t e = cudaMemcpyAsync(x.dst, x.src, x.bytes, out ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, s);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaStreamSynchronize(s);
   }
 
   static bool finite_doubles(const char* p, size_t bytes) {
@@ -111,8 +121,8 @@ class Staging {
     }
     const int n = (int)pieces.size();
     if (n == 0) return out ? cudaStreamSynchronize(s) : cudaSuccess;
-    cudaError_t e = ensure(n);
-    if (e != cudaSuccess) return e;
+    ensure(n);
+    if (have_ == 0) return copy_plain(spans, s, out, bad);
     const int slots = std::min(n, have_);
     std::vector<std::atomic<int>> queued(slots);
     for (auto& q : queued) q.store(-1);

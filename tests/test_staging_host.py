@@ -1,0 +1,130 @@
+"""The pinned staging memory's host side (``csrc/krr_staging.h``) against a CUDA runtime of the test's own (CPU).
+
+The header is compiled with a ``cuda_runtime.h`` whose copies are immediate and whose pinned
+allocations and event creations succeed a given number of times.
+"""
+
+from __future__ import annotations
+
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+RUNTIME = r"""
+#pragma once
+#include <atomic>
+#include <cstdlib>
+#include <cstring>
+#include <thread>
+#include <vector>
+enum cudaError_t { cudaSuccess = 0, cudaErrorMemoryAllocation = 2, cudaErrorUnknown = 999 };
+enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
+enum cudaMemoryType { cudaMemoryTypeUnregistered = 0, cudaMemoryTypeHost = 1 };
+struct cudaPointerAttributes { cudaMemoryType type; };
+using cudaStream_t = int;
+using cudaEvent_t = int;
+constexpr unsigned cudaHostAllocDefault = 0, cudaEventDisableTiming = 2;
+namespace fake {
+inline std::atomic<int> allocs{1 << 30}, events{1 << 30}, made{0}, freed{0}, direct{0};
+inline std::vector<char*> blocks;
+inline bool pinned(const void* p) {
+  for (char* b : blocks)
+    if (p >= b && p < b + ((size_t)4 << 20)) return true;
+  return false;
+}
+}  // namespace fake
+inline cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+  if (fake::allocs.fetch_sub(1) <= 0) return cudaErrorMemoryAllocation;
+  *p = std::malloc(n);
+  fake::blocks.push_back(static_cast<char*>(*p));
+  ++fake::made;
+  return cudaSuccess;
+}
+inline cudaError_t cudaFreeHost(void*) { return ++fake::freed, cudaSuccess; }
+inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+  return fake::events.fetch_sub(1) <= 0 ? cudaErrorMemoryAllocation : (*e = 1, cudaSuccess);
+}
+inline cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+inline cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+inline cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+inline cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  if (!fake::pinned(d) && !fake::pinned(s)) ++fake::direct;
+  std::memcpy(d, s, n);
+  return cudaSuccess;
+}
+inline cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
+  a->type = cudaMemoryTypeUnregistered;
+  return cudaSuccess;
+}
+inline cudaError_t cudaGetLastError() { return cudaSuccess; }
+inline cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+"""
+
+PROGRAM = r"""
+#include <cstdio>
+#include <limits>
+#include "krr_staging.h"
+
+// Arrays of the sizes given (in doubles) through `staging`, out and in; prints what arrived.
+static void both_ways(krr_host::Staging& staging, const std::vector<size_t>& sizes) {
+  std::vector<std::vector<double>> a, b, c;
+  std::vector<krr_host::CopySpan> out, in;
+  for (size_t n : sizes) {
+    a.emplace_back(n);
+    for (size_t i = 0; i < n; ++i) a.back()[i] = 1.0 + (double)(i * 2654435761u % 1000003);
+    b.emplace_back(n, -1.0);
+    c.emplace_back(n, -1.0);
+  }
+  for (size_t k = 0; k < sizes.size(); ++k) {
+    out.push_back({b[k].data(), a[k].data(), sizes[k] * 8});
+    in.push_back({c[k].data(), a[k].data(), sizes[k] * 8});
+  }
+  std::atomic<bool> bad{false};
+  bool ok = staging.out(0, out, 0) == cudaSuccess && staging.in(0, in, 0, &bad) == cudaSuccess && a == b && a == c && !bad;
+  a.back().back() = std::numeric_limits<double>::infinity();
+  ok = ok && staging.in(0, in, 0, &bad) == cudaSuccess && bad;
+  std::printf("ok %d made %d freed %d direct %d\n", (int)ok, (int)fake::made, (int)fake::freed, (int)fake::direct);
+}
+
+int main(int, char** argv) {
+  krr_host::Staging staging;
+  const std::vector<size_t> sizes = {100000, 131072, 131073, 1, 900000, 4500000};
+  fake::allocs = std::atoi(argv[1]);
+  fake::events = std::atoi(argv[2]);
+  both_ways(staging, sizes);
+  return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    folder = tmp_path_factory.mktemp("staging")
+    (folder / "cuda_runtime.h").write_text(RUNTIME)
+    (folder / "staging.cpp").write_text(PROGRAM)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(folder), "-I", str(ROOT / "kerrray_b200" / "csrc"),
+                    str(folder / "staging.cpp"), "-o", str(folder / "staging"), "-pthread"], check=True)
+    return folder / "staging"
+
+
+def _run(program, *args):
+    run = subprocess.run([str(program), *map(str, args)], capture_output=True, text=True, timeout=120)
+    assert run.returncode == 0, run.stderr
+    return run.stdout.split()
+
+
+@pytest.mark.parametrize("allocs,events,direct", [
+    (1000, 1000, False),
+    (3, 1000, False),   # 12 slots of 32
+    (1, 1000, False),
+    (0, 1000, True),    # no pinned memory at all
+    (1000, 6, False),   # the second group's events fail
+    (1000, 2, True),
+])
+def test_transfers_do_with_the_pinned_memory_there_is(program, allocs, events, direct):
+    words = _run(program, allocs, events)
+    assert words[:2] == ["ok", "1"]
+    assert (int(words[words.index("direct") + 1]) > 0) == direct
