@@ -16,8 +16,10 @@
 
 #include <algorithm>
 #include <atomic>
+#include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <thread>
 #include <vector>
 
@@ -180,16 +182,33 @@ class Staging {
       for (int i = 0; i < slots && idle(i); ++i) queue_piece(i);
     const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
     const int threads = (int)std::min<size_t>((size_t)std::min(kThreads, hw), 1 + total / kBytesPerThread);
+    // The workers of an out() sleep until the first piece has arrived: a trace of any length may run
+    // ahead of the copies, and a thread that waits for an event keeps a core busy.
+    std::mutex gate;
+    std::condition_variable opened;
+    bool open = !out;
     std::vector<std::thread> pool;
     for (int t = 1; t < threads; ++t) {
       try {
         pool.emplace_back([&] {
+          {
+            std::unique_lock<std::mutex> lk(gate);
+            opened.wait(lk, [&] { return open; });
+          }
           cudaSetDevice(device);
           work();
         });
       } catch (...) {
         break;  // no more threads to be had: the others do the work
       }
+    }
+    if (out) {
+      wait_slot(0);
+      {
+        std::lock_guard<std::mutex> lk(gate);
+        open = true;
+      }
+      opened.notify_all();
     }
     work();
     for (auto& t : pool) t.join();

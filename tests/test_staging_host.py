@@ -1,7 +1,8 @@
 """The pinned staging memory's host side (``csrc/krr_staging.h``) against a CUDA runtime of the test's own (CPU).
 
-The header is compiled with a ``cuda_runtime.h`` whose copies are immediate and whose pinned
-allocations and event creations succeed a given number of times.
+The header is compiled with a ``cuda_runtime.h`` whose copies are immediate, whose pinned
+allocations and event creations succeed a given number of times, and whose stream can be held (a
+kernel running ahead of the copies): events then complete when it is let go.
 """
 
 from __future__ import annotations
@@ -15,6 +16,7 @@ from conftest import ROOT
 RUNTIME = r"""
 #pragma once
 #include <atomic>
+#include <chrono>
 #include <cstdlib>
 #include <cstring>
 #include <thread>
@@ -24,15 +26,24 @@ enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
 enum cudaMemoryType { cudaMemoryTypeUnregistered = 0, cudaMemoryTypeHost = 1 };
 struct cudaPointerAttributes { cudaMemoryType type; };
 using cudaStream_t = int;
-using cudaEvent_t = int;
+struct FakeEvent { std::atomic<bool> recorded{false}; };
+using cudaEvent_t = FakeEvent*;
 constexpr unsigned cudaHostAllocDefault = 0, cudaEventDisableTiming = 2;
 namespace fake {
-inline std::atomic<int> allocs{1 << 30}, events{1 << 30}, made{0}, freed{0}, direct{0};
+inline std::atomic<int> allocs{1 << 30}, events{1 << 30}, made{0}, freed{0}, direct{0}, waiting{0}, most_waiting{0};
+inline std::atomic<bool> held{false};
 inline std::vector<char*> blocks;
 inline bool pinned(const void* p) {
   for (char* b : blocks)
     if (p >= b && p < b + ((size_t)4 << 20)) return true;
   return false;
+}
+inline void wait() {
+  const int n = ++waiting;
+  int seen = most_waiting;
+  while (n > seen && !most_waiting.compare_exchange_weak(seen, n)) {}
+  while (held) std::this_thread::sleep_for(std::chrono::milliseconds(1));
+  --waiting;
 }
 }  // namespace fake
 inline cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
@@ -44,12 +55,15 @@ inline cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
 }
 inline cudaError_t cudaFreeHost(void*) { return ++fake::freed, cudaSuccess; }
 inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
-  return fake::events.fetch_sub(1) <= 0 ? cudaErrorMemoryAllocation : (*e = 1, cudaSuccess);
+  return fake::events.fetch_sub(1) <= 0 ? cudaErrorMemoryAllocation : (*e = new FakeEvent, cudaSuccess);
 }
-inline cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-inline cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-inline cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-inline cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+inline cudaError_t cudaEventDestroy(cudaEvent_t e) { return delete e, cudaSuccess; }
+inline cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { return e->recorded = true, cudaSuccess; }
+inline cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+  if (e->recorded) fake::wait();
+  return cudaSuccess;
+}
+inline cudaError_t cudaStreamSynchronize(cudaStream_t) { return fake::wait(), cudaSuccess; }
 inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
   if (!fake::pinned(d) && !fake::pinned(s)) ++fake::direct;
   std::memcpy(d, s, n);
@@ -89,12 +103,25 @@ static void both_ways(krr_host::Staging& staging, const std::vector<size_t>& siz
   std::printf("ok %d made %d freed %d direct %d\n", (int)ok, (int)fake::made, (int)fake::freed, (int)fake::direct);
 }
 
-int main(int, char** argv) {
+int main(int argc, char** argv) {
   krr_host::Staging staging;
   const std::vector<size_t> sizes = {100000, 131072, 131073, 1, 900000, 4500000};
-  fake::allocs = std::atoi(argv[1]);
-  fake::events = std::atoi(argv[2]);
-  both_ways(staging, sizes);
+  if (argc > 2) {
+    fake::allocs = std::atoi(argv[1]);
+    fake::events = std::atoi(argv[2]);
+    both_ways(staging, sizes);
+  } else {
+    fake::held = true;
+    std::thread kernel([] {
+      std::this_thread::sleep_for(std::chrono::milliseconds(300));
+      std::printf("waiting %d\n", (int)fake::most_waiting);
+      fake::held = false;
+    });
+    std::vector<double> from(4000000, 2.5), to(4000000, 0.0);
+    const bool ok = staging.out(0, {{to.data(), from.data(), from.size() * 8}}, 0) == cudaSuccess && to == from;
+    kernel.join();
+    std::printf("ok %d\n", (int)ok);
+  }
   return 0;
 }
 """
@@ -128,3 +155,8 @@ def test_transfers_do_with_the_pinned_memory_there_is(program, allocs, events, d
     words = _run(program, allocs, events)
     assert words[:2] == ["ok", "1"]
     assert (int(words[words.index("direct") + 1]) > 0) == direct
+
+
+def test_one_thread_waits_for_the_trace(program):
+    """A 32 MB result behind a kernel: twelve threads may copy, one may wait for the kernel's end."""
+    assert _run(program) == ["waiting", "1", "ok", "1"]
