@@ -3,13 +3,17 @@
 //
 // The driver copies pageable memory through a buffer of its own, one thread, one array after the
 // other, and the pages of a freshly allocated result are faulted in by that thread as well: 5-6 GB/s
-// on this host, so that a batch of 90k rays (11.5 MB of results) spent 3.5 ms on the way back and 2.9M
-// photons (189 MB in, 377 MB out) 80 ms, more than their traces.  Here the transfers are cut into
-// pieces that go through a ring of pinned slots at the bus's rate, while worker threads move the
-// pieces between the slots and the arrays (and take the page faults in parallel).  Small transfers
-// use the calling thread only: one wait for all arrays instead of one per array.
-// 300^2 rays end to end 13.0 -> 11.4 ms (kernel 9.4), 100k float32 rays 5.9 -> 4.6 ms (2.5), 2.9M
-// photons with a host Y0 115 -> 61 ms (trace 41); 6, 12 and 16 threads on a 16-core host within 3 %.
+// where they are, 17 GB/s where the memory is reused, with a wait per array.  Here the transfers are
+// cut into pieces that go through a ring of pinned slots at the bus's rate (50 GB/s), while worker
+// threads move the pieces between the slots and the arrays (and take the page faults in parallel), and
+// one wait serves all arrays.  End to end, fast64 at rtol 1e-6, medians, with the driver's copies and
+// with these: 128^2 photons (2 MB of results) 1.10 and 0.86 ms, 256^2 (8 MB) 1.77 and 1.65, 300^2
+// 2.23 and 1.92, 400^2 3.48 and 2.87, 700^2 9.24 and 6.00, 1000^2 42.6 and 14.4.
+// Threads: one below 8 MB, two to 16 MB, one per 2 MB beyond, at most 12.  A thread per 2 MB from the
+// start made calls of 5 to 16 MB vary from call to call, by up to two (mixed precision, 256^2: 1.04 to
+// 1.95 ms, median 1.48-1.65; by this rule 1.30-1.37, by the driver 1.43-1.48), whether the workers were
+// new, waiting or joined; large transfers gain from all of them (92 MB of camera states at best 19.5 ms
+// by the driver, 3.8 by 12 threads, 5.3 by 6; a 1000^2 image 11.6 ms by 12, 13.1 by 6).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -48,7 +52,7 @@ class Staging {
  public:
   static constexpr size_t kSlotBytes = (size_t)1 << 20;
   static constexpr int kSlots = 32, kGroup = 4;
-  static constexpr size_t kBytesPerThread = (size_t)1 << 21;  // a thread more per 2 MB, up to kThreads
+  static constexpr size_t kFew = (size_t)1 << 24;  // a transfer below this takes one thread or two
   static constexpr int kThreads = 12;
 
   // Device to host arrays, after what `s` holds now; returns when every byte is in place.
@@ -123,6 +127,8 @@ class Staging {
     }
     const int n = (int)pieces.size();
     if (n == 0) return out ? cudaStreamSynchronize(s) : cudaSuccess;
+    // One array, and no values to check on the way: the driver's copy overlaps its own staging.
+    if (!bad && spans.size() == 1 && total < kFew) return copy_plain(spans, s, out, nullptr);
     ensure(n);
     if (have_ == 0) return copy_plain(spans, s, out, bad);
     const int slots = std::min(n, have_);
@@ -181,7 +187,8 @@ class Staging {
     if (out)
       for (int i = 0; i < slots && idle(i); ++i) queue_piece(i);
     const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-    const int threads = (int)std::min<size_t>((size_t)std::min(kThreads, hw), 1 + total / kBytesPerThread);
+    const int threads = (int)std::min<size_t>((size_t)std::min(kThreads, hw),
+                                              total < kFew ? 1 + total / (kFew / 2) : total / (kFew / 8));
     // The workers of an out() sleep until the first piece has arrived: a trace of any length may run
     // ahead of the copies, and a thread that waits for an event keeps a core busy.
     std::mutex gate;
