@@ -55,12 +55,10 @@ class Backend(Protocol):
 
 
 def _validate_batch(Y0: ArrayLike) -> np.ndarray:
-    # A private copy: the library reads the rows after the GIL is released, so a caller's thread that
-    # writes to its array must not reach rows that were, or are about to be, checked.
-    arr = np.array(Y0, dtype=np.float64, order="C")
+    arr = np.asarray(Y0, dtype=np.float64)
     if arr.ndim != 2 or arr.shape[1] != STATE_SIZE:
         raise ValueError(f"Y0 must have shape (N, {STATE_SIZE}), got {arr.shape}")
-    return arr  # the library checks that every value is finite
+    return np.ascontiguousarray(arr)  # the library reads it once and checks that what it read is finite
 
 
 def _result_type():

@@ -1097,18 +1097,30 @@ int krr_integrate_batch(int device, double mass, double spin, const double* Y0, 
   if (rc) return rc;
   if (n < 0) return fail(KRR_ERR_INVALID, "n must be >= 0, got %lld", (long long)n);
   if (!out || (n > 0 && (!Y0 || !out->Y || !out->state))) return fail(KRR_ERR_INVALID, "Y0, Y and state must not be NULL");
-  // Before the device is looked for, as the reference's check comes before its backend's work.
-  if (n > 0 && !all_finite_parallel(Y0, (size_t)n * 8)) return fail(KRR_ERR_INVALID, "Y0 must be finite");
   Context* c = nullptr;
   rc = get_context(device, &c);
+  // Without a device an invalid Y0 is still the error, as the reference's check comes before its
+  // backend's work.
+  if (rc && n > 0 && !all_finite_parallel(Y0, (size_t)n * 8)) return fail(KRR_ERR_INVALID, "Y0 must be finite");
   if (rc) return rc;
   std::lock_guard<std::mutex> lk(c->mu);
   KRR_CUDA(cudaSetDevice(device));
   if (n > 0) {
-    KRR_CUDA(c->buf[B_Y0].ensure((size_t)n * 8 * sizeof(double)));
-    rc = copy_in(c, c->buf[B_Y0].p, Y0, (size_t)n * 8 * sizeof(double), c->stream, nullptr);
-    if (rc) return rc;
-    const double* d_Y0 = static_cast<const double*>(c->buf[B_Y0].p);
+    // The caller's rows are read once, and what was read is checked (a pageable Y0 in the staging
+    // memory, a pinned one on the device) before it is traced: a caller's thread that writes to them
+    // meanwhile cannot bring in rows that were not checked.
+    const double* d_Y0 = nullptr;
+    if (host_pinned(Y0)) {
+      rc = upload_y0(c, Y0, n, &d_Y0);
+      if (rc) return rc;
+    } else {
+      std::atomic<bool> bad{false};
+      KRR_CUDA(c->buf[B_Y0].ensure((size_t)n * 8 * sizeof(double)));
+      rc = copy_in(c, c->buf[B_Y0].p, Y0, (size_t)n * 8 * sizeof(double), c->stream, &bad);
+      if (rc) return rc;
+      if (bad.load()) return fail(KRR_ERR_INVALID, "Y0 must be finite");
+      d_Y0 = static_cast<const double*>(c->buf[B_Y0].p);
+    }
     krr_result dev;
     rc = device_results(c, n, out, options->disk_plane != 0, &dev);
     if (rc) return rc;

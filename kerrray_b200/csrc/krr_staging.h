@@ -23,7 +23,9 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -59,8 +61,8 @@ class Staging {
   cudaError_t out(int device, const std::vector<CopySpan>& spans, cudaStream_t s) {
     return run(device, spans, s, true, nullptr);
   }
-  // Host arrays (of doubles) to the device on `s`; returns when the host arrays have been read and
-  // every copy is queued.  *bad is set where a value is not finite.
+  // Host arrays (of doubles) to the device on `s`; returns when the host arrays have been read, once,
+  // and every copy is queued.  *bad (nullable) is set where a value that was read is not finite.
   cudaError_t in(int device, const std::vector<CopySpan>& spans, cudaStream_t s, std::atomic<bool>* bad) {
     return run(device, spans, s, false, bad);
   }
@@ -91,12 +93,26 @@ class Staging {
     }
   }
 
-  // Without any slot: the driver's own copies of pageable memory.
+  // Without any slot: the driver's own copies of pageable memory.  What is checked goes through memory
+  // of this call's own, so that the values copied are the ones checked.
   static cudaError_t copy_plain(const std::vector<CopySpan>& spans, cudaStream_t s, bool out, std::atomic<bool>* bad) {
+    std::unique_ptr<char[]> own(bad ? new (std::nothrow) char[kSlotBytes] : nullptr);
+    if (bad && !own) return cudaErrorMemoryAllocation;
     for (const CopySpan& x : spans) {
-      if (bad && !finite_doubles(static_cast<const char*>(x.src), x.bytes)) bad->store(true);
-      const cudaError_t e = cudaMemcpyAsync(x.dst, x.src, x.bytes, out ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, s);
-      if (e != cudaSuccess) return e;
+      const size_t step = bad ? kSlotBytes : x.bytes;
+      for (size_t o = 0; o < x.bytes; o += step) {
+        const size_t n = std::min(step, x.bytes - o);
+        const char* src = static_cast<const char*>(x.src) + o;
+        if (bad) {
+          std::memcpy(own.get(), src, n);
+          if (!finite_doubles(own.get(), n)) bad->store(true);
+          src = own.get();
+        }
+        cudaError_t e = cudaMemcpyAsync(static_cast<char*>(x.dst) + o, src, n,
+                                        out ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess && bad) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return e;
+      }
     }
     return cudaStreamSynchronize(s);
   }

@@ -18,6 +18,7 @@ RUNTIME = r"""
 #pragma once
 #include <atomic>
 #include <chrono>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <thread>
@@ -34,6 +35,7 @@ namespace fake {
 inline std::atomic<int> allocs{1 << 30}, events{1 << 30}, made{0}, freed{0}, direct{0}, workers{0}, waiting{0}, most_waiting{0};
 inline std::atomic<bool> held{false};
 inline std::vector<char*> blocks;
+inline std::vector<double>* poisoned = nullptr;  // another thread's array: it turns to NaN when the first copy is queued
 inline bool pinned(const void* p) {
   for (char* b : blocks)
     if (p >= b && p < b + ((size_t)4 << 20)) return true;
@@ -66,6 +68,8 @@ inline cudaError_t cudaEventSynchronize(cudaEvent_t e) {
 }
 inline cudaError_t cudaStreamSynchronize(cudaStream_t) { return fake::wait(), cudaSuccess; }
 inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  if (fake::poisoned)
+    for (double& x : *fake::poisoned) x = NAN;
   if (!fake::pinned(d) && !fake::pinned(s)) ++fake::direct;
   std::memcpy(d, s, n);
   return cudaSuccess;
@@ -107,7 +111,16 @@ static void both_ways(krr_host::Staging& staging, const std::vector<size_t>& siz
 int main(int argc, char** argv) {
   krr_host::Staging staging;
   const std::vector<size_t> sizes = {100000, 131072, 131073, 1, 900000, 4500000};
-  if (argc > 3) {  // the workers and the driver's copies of a transfer of argv[2] arrays of argv[3] doubles
+  if (argc > 4) {  // one checked array, written to while it is copied
+    fake::allocs = std::atoi(argv[4]);
+    std::vector<double> a(std::atoll(argv[3]), 1.0), b(a.size(), 0.0);
+    fake::poisoned = &a;
+    std::atomic<bool> bad{false};
+    const bool ok = staging.in(0, {{b.data(), a.data(), a.size() * 8}}, 0, &bad) == cudaSuccess;
+    bool finite = true;
+    for (double x : b) finite = finite && std::isfinite(x);
+    std::printf("ok %d sound %d\n", (int)ok, (int)(bad || finite));
+  } else if (argc > 3) {  // the workers and the driver's copies of a transfer of argv[2] arrays of argv[3] doubles
     std::vector<std::vector<double>> a(std::atoi(argv[2]), std::vector<double>(std::atoll(argv[3]), 1.0)), b = a;
     std::vector<krr_host::CopySpan> spans;
     for (size_t k = 0; k < a.size(); ++k) spans.push_back({b[k].data(), a[k].data(), a[k].size() * 8});
@@ -188,3 +201,10 @@ def test_threads_by_the_size_of_a_transfer(program, way, arrays, doubles, worker
     """A thread more costs a short call more than it saves; workers that find no piece left count as well."""
     most = min(12, os.cpu_count() or 1) - 1
     assert _run(program, way, arrays, doubles) == ["ok", "1", "workers", str(min(workers, most)), "direct", str(direct)]
+
+
+@pytest.mark.parametrize("doubles", [1000, 131072])
+@pytest.mark.parametrize("allocs", [0, 1000])
+def test_values_copied_are_the_ones_checked(program, doubles, allocs):
+    """With and without pinned memory the caller's array is read once."""
+    assert _run(program, 2, 1, doubles, allocs) == ["ok", "1", "sound", "1"]
