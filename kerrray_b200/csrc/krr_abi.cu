@@ -435,6 +435,16 @@ const krr::Variant* variants_for(int32_t precision, const krr_options* o, int* c
   return krr::fast_variants(precision == KRR_PREC_MIXED, rk4, count);
 }
 
+// A launch variant that exists (no device is touched).
+int check_variant(int32_t precision, const krr_options* o, const krr_launch* l) {
+  int count = 0;
+  const krr::Variant* vs = variants_for(precision, o, &count);
+  if (!vs || count < 1) return fail(KRR_ERR_UNSUPPORTED, "no persistent kernel for this precision/method");
+  const int idx = (l && l->variant > 0) ? l->variant : 0;
+  if (idx >= count) return fail(KRR_ERR_INVALID, "launch variant %d out of range [0, %d)", idx, count);
+  return KRR_OK;
+}
+
 // The launch shape a caller asked for or, with none of variant, blocks_per_sm and refill_threshold
 // set, the library's for `total` photons (each measured on the B200; the results never differ).
 // With `lanes` the resident lanes of variant 0, the shape without a register cap:
@@ -457,11 +467,10 @@ const krr::Variant* variants_for(int32_t precision, const krr_options* o, int* c
 //   unrolled: 21.4 ms at 1, 16.0 at 4, 14.3 at 8, 13.8 at 12 (300^2: 5.2, 4.8, 4.6, 4.6).
 int persistent_shape(int device, int32_t precision, const krr_options* o, const krr_launch* l, long long total,
                      LaunchShape& s) {
-  int count = 0;
+  int rc = check_variant(precision, o, l);
+  if (rc) return rc;
+  int count = 0, idx = (l && l->variant > 0) ? l->variant : 0;
   const krr::Variant* vs = variants_for(precision, o, &count);
-  if (!vs || count < 1) return fail(KRR_ERR_UNSUPPORTED, "no persistent kernel for this precision/method");
-  int idx = (l && l->variant > 0) ? l->variant : 0;
-  if (idx >= count) return fail(KRR_ERR_INVALID, "launch variant %d out of range [0, %d)", idx, count);
   const bool chosen = l && (l->variant > 0 || l->blocks_per_sm > 0 || l->refill_threshold > 0);
   const long long sms = sm_count_of(device);
   int occ = vs[idx].occupancy();

@@ -18,6 +18,7 @@ int make_frame(double mass, double spin, const krr_camera* c, krr::Frame& F);
 krr::Outputs to_outputs(const krr_result* r);
 const krr::Variant* variants_for(int32_t precision, const krr_options* o, int* count);
 int sm_count_of(int device);
+int check_variant(int32_t precision, const krr_options* o, const krr_launch* l);
 
 // The persistent kernel's launch: compiled shape, blocks, idle lanes before a warp refills; and
 // whether one photon per thread in blocks of `plain_block` threads is the faster launch (0: no).

@@ -88,6 +88,8 @@ extern "C" int krr_trace_images_noalloc(int device, const krr_image* images, int
   }
   int rc = check_precision(precision, &images[0].options);
   if (rc) return rc;
+  rc = check_variant(precision, &images[0].options, launch);
+  if (rc) return rc;
   if (cudaSetDevice(device) != cudaSuccess) return fail(KRR_ERR_NO_DEVICE, "cannot select device %d", device);
   LaunchShape shape{};
   rc = persistent_shape(device, precision, &images[0].options, launch, total, shape);
