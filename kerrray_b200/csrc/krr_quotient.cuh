@@ -88,7 +88,7 @@ __device__ __forceinline__ double quotient_any(double a, double b) {
   const unsigned ha = (unsigned)__double2hiint(a) & 0x7fffffffu, hb = (unsigned)__double2hiint(b) & 0x7fffffffu;
   const double q = quotient(a, b);
   const bool ok = hb - 0x26f00000u < 0x32000000u && fraction_gap(b) != 0u &&
-                  (a == 0.0 || ha - 0x07b00000u < 0x70800000u);
+                  (a == 0.0 || ha - 0x20b00000u < 0x3e800000u);
   return ok ? q : quotient_ieee(a, b);
 }
 
