@@ -106,10 +106,9 @@ krr::Params make_params(double mass, double spin, const krr_options* o) {
   P.max_steps = o->max_steps;
   P.guard = max_attempts(o);
   P.rk4 = o->method == 1;
-  // The ranges under which the reference order's branch-free divisions neither overflow nor
-  // underflow (RefMode::metric, attempt); other scales divide by IEEE division.
-  const double big = std::ldexp(1.0, 60), small = std::ldexp(1.0, -60);
-  P.div_ok = m >= small && m <= big && (a == 0.0 || std::fabs(a) >= small) && o->atol >= std::ldexp(1.0, -400);
+  // The masses and spins for which the reference order's branch-free divisions neither overflow nor
+  // underflow (RefMode::metric_straight); with others it divides by IEEE division.
+  P.div_ok = m >= std::ldexp(1.0, -50) && m <= std::ldexp(1.0, 60) && (a == 0.0 || std::fabs(a) >= std::ldexp(1.0, -120));
   P.disk = o->disk_plane != 0;
   P.r_plus = outer_horizon(m, a);
   P.f_mass = (float)m;
@@ -502,8 +501,9 @@ int persistent_shape(int device, int32_t precision, const krr_options* o, const 
 }
 
 // Four lanes per ray in reference order (krr_quad.cuh): up to two warps of eight rays per scheduler.
-bool quad_fits(int device, int32_t precision, const krr_options* o, bool events, long long n) {
-  return precision == KRR_PREC_REFERENCE && o->dtype == 0 && o->method == 0 && !events &&
+// Not where every step would leave the branch-free divisions (div_ok false) and be done by each lane.
+bool quad_fits(int device, int32_t precision, const krr_options* o, bool events, bool div_ok, long long n) {
+  return precision == KRR_PREC_REFERENCE && o->dtype == 0 && o->method == 0 && !events && div_ok &&
          n <= (long long)sm_count_of(device) * 4 * 16;
 }
 
@@ -652,9 +652,12 @@ int prepare_pipeline(int device, const krr_image* images, int n_images, long lon
   if (shape.plain_block > 0 && !p.retrace && !p.plain) {
     p.plain = true;
     p.plain_block = shape.plain_block;
-    bool events = false;
-    for (int k = 0; k < n_images; ++k) events = events || images[k].options.disk_plane;
-    p.quad = quad_fits(device, precision, o0, events, total);
+    bool events = false, div_ok = true;
+    for (int k = 0; k < n_images; ++k) {
+      events = events || images[k].options.disk_plane;
+      div_ok = div_ok && make_params(images[k].mass, images[k].spin, &images[k].options).div_ok;
+    }
+    p.quad = quad_fits(device, precision, o0, events, div_ok, total);
   }
   p.main_v = shape.v;
   p.main.images = p.w.images;
@@ -1090,7 +1093,7 @@ int krr_integrate_batch_device(int device, double mass, double spin, const doubl
   a.o = to_outputs(d_out);
   a.q = nullptr;
   a.rtol_max = options->rtol;
-  a.quad = quad_fits(device, precision, options, options->disk_plane != 0, n);
+  a.quad = quad_fits(device, precision, options, options->disk_plane != 0, a.P.div_ok, n);
   KRR_CUDA(launch_plain(precision, options, a, 32, static_cast<cudaStream_t>(stream)));
   return KRR_OK;
 }
@@ -1169,7 +1172,7 @@ int krr_integrate_batch(int device, double mass, double spin, const double* Y0, 
       a.n = n;
       a.o = to_outputs(&dev);
       a.rtol_max = options->rtol;
-      a.quad = quad_fits(device, precision, options, options->disk_plane != 0, n);
+      a.quad = quad_fits(device, precision, options, options->disk_plane != 0, a.P.div_ok, n);
       KRR_CUDA(launch_plain(precision, options, a, shape.plain_block, c->stream));
     } else {
       krr::PersistArgs a{};

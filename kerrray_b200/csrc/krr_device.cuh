@@ -75,7 +75,7 @@ struct Params {
   double r_plus;  // outer horizon M + sqrt(M^2 - a^2)
   long long max_steps, guard;
   short rk4;     // 0: Dormand-Prince 5(4), 1: fixed-step RK4
-  short div_ok;  // the scales allow the branch-free divisions (RefMode::metric, attempt); set by make_params
+  short div_ok;  // mass and spin allow the branch-free divisions (RefMode::metric_straight); set by make_params
   int disk;      // disk-plane event enabled
   // FP32 copies for the mixed mode's stages (rounded once on the host).
   float f_mass, f_a, f_a2;
@@ -190,7 +190,7 @@ struct RefMode {
     double sig, sd, sd2, sig2, sds2, sig2s2, sig2s4;            // denominators
     double n0, n1, dlt, n4, n5, n6, n7, n8, n9, n10, n11, n12, n13, n14;  // numerators (n9: of a2 sd_r / sd2)
     double m14;                                                  // numerator of a2 sd_th / sd2
-    double s2;
+    double s2, r2;
   };
   __device__ __forceinline__ static Terms terms(const Params& P, double r, double s, double c, double sin2th) {
     const double m = P.mass, a2 = P.a2;
@@ -211,6 +211,7 @@ struct RefMode {
     const double sd_th = sig_th * dlt;
     const double sig2 = sig * sig;
     t.s2 = s2;
+    t.r2 = r2;
     t.sig = sig;
     t.sd = sd;
     t.sd2 = sd * sd;
@@ -265,11 +266,12 @@ struct RefMode {
     return q;
   }
 
-  // The 15 terms without a branch.  The branch-free quotients hold their
-  // values while nothing overflows or underflows: with sin^2, Sigma and Sigma Delta in
-  // [2^-120, 2^120] and the mass and spin in [2^-60, 2^60] (or spin 0; P.div_ok) every denominator
-  // lies in [2^-480, 2^480], and every numerator is 0 or in [2^-700, 2^700] (products of at most six
-  // such factors; a difference that is not 0 is at least 2^-53 of its terms).  The sines and the
+  // The 15 terms without a branch.  The branch-free quotients hold their values while nothing overflows
+  // or underflows: with r^2 in [2^-100, 2^120), sin^2 in [2^-120, 2^120), Sigma Delta in [2^-200, 2^240),
+  // the mass in [2^-50, 2^60] and the spin 0 or at least 2^-120 (P.div_ok) every denominator lies in
+  // [2^-440, 2^480], every numerator is 0 or at least 2^-933 (a difference that is not 0 is at least 2^-54
+  // of its terms), and every quotient in 2^+-900.  That is any tolerance, any spin down to 1e-36 M and
+  // lengths from 1e-15 to 1e18: a hole in metres, centimetres or parsecs.  The sines and the
   // cosine are the compiler's, told that the angle is moderate: their branch to the reduction of
   // large arguments is then left out, and the same values come without it (a 64^2 image 2.35 ->
   // 2.22 ms with the accepted steps' three divisions branch-free as well).
@@ -301,15 +303,21 @@ struct RefMode {
     g[12] = quotient(t.n12, i_sig2);
     g[13] = quotient(t.n13, i_sig2);
     g[14] = quotient(t.n14, t.sig2s4) + quotient(t.m14, i_sd2);
-    return near && gap != 0u && P.div_ok && moderate(t.s2) && moderate(t.sig) && moderate(t.sd);
+    // (P.div_ok holds wherever this is called; without it in the test the compiler orders the unrolled
+    // stages differently and they take 4 to 8 % longer.)
+    return near && gap != 0u && P.div_ok && in_range(t);
+  }
+  __device__ __forceinline__ static bool in_range(const Terms& t) {
+    return within<-120, 120>(t.s2) && within<-100, 120>(t.r2) && within<-200, 240>(t.sd);
   }
 
-  // f (6 integrated components) at state (r, th, pr, pth) with constants (pt, pph).  STRAIGHT: tr.ok
-  // is cleared where the values must not be used.
+  // f (6 integrated components) at state (r, th, pr, pth) with constants (pt, pph).  STRAIGHT (only with
+  // P.div_ok): tr.ok is cleared where the values must not be used.
   template <bool STRAIGHT = false>
   __device__ static void rhs(const Params& P, S r, S th, S pt, S pr, S pth, S pph, K f[NV], Trig& tr) {
     double g64[15];
-    const bool ok = metric_straight(P, (double)r, (double)th, g64, tr);
+    bool ok = false;
+    if (STRAIGHT || P.div_ok) ok = metric_straight(P, (double)r, (double)th, g64, tr);
     if constexpr (STRAIGHT) {
       tr.ok = tr.ok && ok;
     } else if (!ok) {
@@ -1243,7 +1251,8 @@ __device__ __forceinline__ void dp_stages(const Params& P, const Ray<M>& ry, typ
     dp_stages_loop<M>(P, ry, h, k6, yn, esum, tr);
   } else if constexpr (M::kStraight) {
     tr.ok = true;
-    dp_stages_scalar<M, RK4>(P, ry, h, k6, yn, esum, tr);
+    if (M::kFused || P.div_ok) dp_stages_scalar<M, RK4>(P, ry, h, k6, yn, esum, tr);
+    else tr.ok = false;  // no step would pass
     if (!tr.ok) {
       StepStart<M> a;
 #pragma unroll
@@ -1321,20 +1330,19 @@ __device__ __forceinline__ void attempt(const Params& P, Ray<M>& ry, double* __r
       // instead of taking the square root (the step factor is a power of en^2 as well).
       N q[NV];
       if constexpr (!M::kFused && sizeof(N) == 8) {
-        // Six independent IEEE quotients.  Branch-free (quotient) where every scale allows it: at
-        // most 2^400 here and at least atol >= 2^-400 (P.div_ok).  A numerator too small for an
-        // exact residual (below 2^-960) gives |v| < 2^-550 either way and v^2 = 0.
+        // Six independent IEEE quotients.  Branch-free (quotient) where every scale lies in
+        // [2^-400, 2^400): a numerator too small for an exact residual (below 2^-960) then gives
+        // |v| < 2^-550 either way and v^2 = 0, one too large for its quotient a norm that is not finite.
         double e[NV], scale[NV];
-        unsigned gap = 0xffffffffu;
-        int top = 0;
+        unsigned gap = 0xffffffffu, top = 0u;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
           e[i] = h * esum[i];
           scale[i] = P.atol + P.rtol * py_max(fabs(ry.y[i]), fabs(yn[i]));
           gap = min(gap, fraction_gap(scale[i]));
-          top = max(top, __double2hiint(scale[i]));
+          top = max(top, (unsigned)__double2hiint(scale[i]) - 0x26f00000u);  // from 2^-400
         }
-        if (!(gap != 0u && top < 0x58f00000 && P.div_ok)) {  // 2^400
+        if (!(gap != 0u && top < 0x32000000u)) {
           const Six v = quotients_ieee(Six{{e[0], e[1], e[2], e[3], e[4], e[5]}},
                                        Six{{scale[0], scale[1], scale[2], scale[3], scale[4], scale[5]}});
 #pragma unroll

@@ -72,7 +72,8 @@ struct Quad {
     rejected_before = false;
   }
 
-  // The lane's components of the right-hand side at (r, th, pr, pth) into g; s, c on every lane.
+  // The lane's components of the right-hand side at (r, th, pr, pth) into g; s, c on every lane.  False,
+  // with values that must not be used, outside the branch-free range (P.div_ok holds: quad_fits).
   __device__ __forceinline__ bool rhs(const Params& P, double r, double th, double pr, double pth, double g[4], double& s,
                                       double& c) const {
     const bool near = fabs(th) < 1000.0;
@@ -102,7 +103,7 @@ struct Quad {
     g[1] = zero ? q3 * pth : 0.0;
     g[2] = zero ? q0 * pt + q1 * pph : 0.0;
     g[3] = zero ? q1 * pt + (axis ? 0.0 : q4) * pph : 0.0;
-    return near && gap != 0u && P.div_ok && moderate(t.s2) && moderate(t.sig) && moderate(t.sd);
+    return near && gap != 0u && M::in_range(t);
   }
 
   // One step attempt (attempt<RefMode<double>, false> without the disk event), by every lane of the

@@ -74,9 +74,10 @@ __device__ __forceinline__ unsigned fraction_gap(double b) {
   return (~(unsigned)__double2hiint(b)) & 0x000fffffu;
 }
 
-// Whether |x| lies in [2^-120, 2^120) (false for NaN and infinities).
-__device__ __forceinline__ bool moderate(double x) {
-  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x38700000u < 0x0f000000u;
+// Whether |x| lies in [2^LO, 2^HI) (false for NaN and infinities).
+template <int LO, int HI>
+__device__ __forceinline__ bool within(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - ((unsigned)(1023 + LO) << 20) < ((unsigned)(HI - LO) << 20);
 }
 
 // a / b for any operands: branch-free in the range where that holds (|b| in [2^-400, 2^400], a 0 or
