@@ -444,6 +444,14 @@ int check_variant(int32_t precision, const krr_options* o, const krr_launch* l) 
   return KRR_OK;
 }
 
+// Threads per block for one photon per thread.  Blocks of one warp spread best over the SMs once warps
+// of other blocks wait for a place; up to 256 photons per SM none does, and blocks of four warps put
+// one on each scheduler.  Blocks of 32 and 128 threads, ms (rtol 1e-6, kernel): reference order, 10k
+// image photons 2.06 and 1.84, 25k random ones 2.59 and 2.42, 30k 2.58 and 2.39, 45k 3.91 and 4.03;
+// fast64, 25k 0.66 and 0.62 (random 0.72 and 0.68), 60k 0.78 and 0.96; mixed, 25k 0.52 and 0.49, 60k
+// 0.56 and 0.65.
+int plain_block(int device, long long n) { return n <= (long long)sm_count_of(device) * 256 ? 128 : 32; }
+
 // The launch shape a caller asked for or, with none of variant, blocks_per_sm and refill_threshold
 // set, the library's for `total` photons (each measured on the B200; the results never differ).
 // With `lanes` the resident lanes of variant 0, the shape without a register cap:
@@ -454,9 +462,7 @@ int check_variant(int32_t precision, const krr_options* o, const krr_launch* l) 
 //   queue wins (fast64, 737k photons of 72 images: 14.5 ms plain, 12.1 queue; one image: the same
 //   either way from 360k photons up), so up to 4 per lane in the fast modes. In reference order the
 //   queue's kernel is the rolled one, which pays off earlier: 40k photons 4.8 ms plain, 6.0 queue;
-//   90k 5.7 and 5.0: up to 1.5 per lane. Blocks of one warp spread best over the SMs, but up to 128
-//   photons per SM blocks of four, which put one warp on each scheduler: 10k photons in reference
-//   order 2.37 ms in blocks of 32, 2.14 of 128; 20k at rtol 1e-9 7.0 and 7.3.
+//   90k 5.7 and 5.0: up to 1.5 per lane (the blocks' size: plain_block).
 // - the queue on that few photons (where a re-trace needs it) takes variant 0, with the shortest
 //   chain per step, on only the blocks it fills: 100^2 in fast64 0.69 -> 0.57 ms.
 // - a longer queue is bound by throughput: variant 1 (fast64 168 registers, 12 warps per SM; mixed
@@ -479,7 +485,7 @@ int persistent_shape(int device, int32_t precision, const krr_options* o, const 
     const long long lanes = sms * std::max(occ, 0) * vs[0].block;
     fits = total <= lanes;
     if (total <= (precision == KRR_PREC_REFERENCE ? lanes + lanes / 2 : 4 * lanes))
-      s.plain_block = total <= sms * 128 ? 128 : 32;
+      s.plain_block = plain_block(device, total);
     if (!fits && count > 1) {
       idx = 1;
       occ = vs[idx].occupancy();
@@ -1094,7 +1100,8 @@ int krr_integrate_batch_device(int device, double mass, double spin, const doubl
   a.q = nullptr;
   a.rtol_max = options->rtol;
   a.quad = quad_fits(device, precision, options, options->disk_plane != 0, a.P.div_ok, n);
-  KRR_CUDA(launch_plain(precision, options, a, 32, static_cast<cudaStream_t>(stream)));
+  // One ray per thread for any n: the queue needs a workspace, which this entry point has not.
+  KRR_CUDA(launch_plain(precision, options, a, plain_block(device, n), static_cast<cudaStream_t>(stream)));
   return KRR_OK;
 }
 
