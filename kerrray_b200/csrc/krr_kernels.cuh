@@ -827,8 +827,8 @@ cudaError_t run_bisect(EdgeArgs a, cudaStream_t s) {
                                         : run_bisect_as<M, MAXT, MINB, false>(a, s);
 }
 
-// The analytic edge radius of every item into a.star (see k_bisect_edges): NaN where the ends'
-// analytic classes are not "captured at lo, escaped at hi", +-infinity where both are the same.
+// The analytic edge radius of every item into a.star (see k_bisect_edges): NaN, which predicts no path,
+// where the ends' analytic classes are not "captured at lo, escaped at hi".
 __global__ void k_edge_predict(EdgeArgs a);
 cudaError_t edge_predict(const EdgeArgs& a, cudaStream_t s);
 

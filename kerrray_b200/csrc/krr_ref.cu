@@ -106,11 +106,7 @@ __global__ void __launch_bounds__(128) k_edge_predict(EdgeArgs a) {
   double lo = a.lo[i], hi = a.hi[i];
   double f_lo = margin(lo), f_hi = margin(hi);
   double star = CUDART_NAN;
-  if (f_lo < 0.0 && f_hi < 0.0) {
-    star = -CUDART_INF;
-  } else if (f_lo >= 0.0 && f_hi >= 0.0) {
-    star = CUDART_INF;
-  } else if (f_lo >= 0.0 && f_hi < 0.0) {
+  if (f_lo >= 0.0 && f_hi < 0.0) {
     int kept = 0;  // the end the last regula falsi step left: -1 hi, +1 lo
     for (int k = 0; k < 14; ++k) {
       const double x = k < 8 ? 0.5 * (lo + hi) : lo + (hi - lo) * (f_lo / (f_lo - f_hi));
