@@ -135,15 +135,18 @@ typedef struct krr_image {
   int64_t pixel_count;
 } krr_image;
 
-/* Launch shape of the persistent kernel (0 = library default / autotuned). */
+/* Launch shape (0 = library default / autotuned).  With plain, variant, blocks_per_sm and
+ * refill_threshold all 0 the library chooses by the number of photons: up to a few per resident
+ * lane one thread (in reference order up to 64 photons per SM, four lanes) per photon without a
+ * queue, in blocks of its own choice, and beyond the persistent kernel in a shape that suits them.
+ * The results do not depend on the shape. */
 typedef struct krr_launch {
   int32_t precision;         /* KRR_PREC_* */
-  int32_t block;             /* threads per block */
+  int32_t block;             /* threads per block with plain = 1 (0: 128; a multiple of 32) */
   int32_t blocks_per_sm;     /* resident blocks per SM (0: as many as fit) */
-  int32_t refill_threshold;  /* idle lanes of a warp before it refills from the queue (0: 1); with
-                                blocks_per_sm, refill_threshold and variant all 0 the library
-                                chooses the three for the number of photons */
-  int32_t plain;             /* 1: one thread per photon, no work queue (the plain kernel) */
+  int32_t refill_threshold;  /* idle lanes of a warp before it refills from the queue (0: 1) */
+  int32_t plain;             /* 1: one thread per photon, no work queue (the plain kernel), whatever
+                                the number of photons; 0: as chosen above, or the work queue */
   int32_t variant;           /* compiled launch shape of the persistent kernel (krr_list_variants) */
   int32_t retrace;           /* KRR_RETRACE_*: settle the pixels a mixed trace could classify
                                 differently with the reference-order FP64 kernel (rk45, float64,
@@ -196,7 +199,9 @@ KRR_API int krr_integrate_batch(int device, double mass, double spin, const doub
 
 /* The same on device buffers (Y0 and every result array on `device`), enqueued on `stream`
  * (a cudaStream_t; NULL = legacy default stream); returns without synchronising.  index
- * (nullable, device) selects rows: ray i integrates Y0[index[i]] and writes row index[i]. */
+ * (nullable, device) selects rows: ray i integrates Y0[index[i]] and writes row index[i].
+ * One ray per thread (or four lanes) for any n: the work queue, which large batches of
+ * krr_integrate_batch run through, needs a workspace. */
 KRR_API int krr_integrate_batch_device(int device, double mass, double spin, const double* d_Y0,
                                const int64_t* d_index, int64_t n, const krr_options* options,
                                int32_t precision, const krr_result* d_out, void* stream);

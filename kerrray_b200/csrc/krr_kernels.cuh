@@ -154,8 +154,8 @@ __global__ void k_trace_plain(const __grid_constant__ Params P, const Image* __r
 // still end unlike its class, it is marked for the reference-order re-trace.  A kernel after the main
 // trace for these three photons of a 1024^2 image took 0.41 ms, the length of their remaining chains
 // with the rest of the GPU idle; traced on in place they end with the others.
-// TRACE_ONE_PER_SCHEDULER -- only the first four warps of a block take photons, the others leave: a
-// block that fills an SM's registers for a few long chains then runs one warp on each scheduler.
+// TRACE_ONE_PER_SCHEDULER -- only the first four warps of a block take photons, the others wait at its
+// end: a block that fills an SM's registers for a few long chains then runs one warp on each scheduler.
 enum : int { TRACE_SPREAD = 1, TRACE_RESUME = 2, TRACE_SKIP_NEAR = 4, TRACE_RESTART = 8, TRACE_ONE_PER_SCHEDULER = 16 };
 
 template <class M>

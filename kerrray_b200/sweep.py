@@ -142,13 +142,15 @@ class ImageSpec:
 
 @dataclass(frozen=True)
 class LaunchConfig:
-    """Launch shape of the persistent kernel. With ``blocks_per_sm``, ``refill_threshold`` and
-    ``variant`` all 0 the library chooses the three for the number of photons."""
+    """Launch shape. With ``plain`` unset and ``blocks_per_sm``, ``refill_threshold`` and ``variant``
+    all 0 the library chooses by the number of photons: few of them run one thread (in reference
+    order four lanes) per photon without a queue, more through the persistent kernel in a shape that
+    suits them. The results do not depend on the shape."""
 
-    block: int = 0            # threads per block of the plain kernel
+    block: int = 0            # threads per block with plain=True
     blocks_per_sm: int = 0    # resident blocks per SM (0 = as many as fit)
     refill_threshold: int = 0  # idle lanes before a warp refills (0 = 1)
-    plain: bool = False       # one thread per photon instead of the work queue
+    plain: bool = False       # one thread per photon, whatever their number
     variant: int = 0          # compiled launch shape of the persistent kernel
     # Settle the pixels a mixed trace could classify differently with the reference-order FP64
     # kernel: 0 off; 1 (RETRACE_EDGE) afterwards, every pixel not ESCAPED or CAPTURED or unlike a
