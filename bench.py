@@ -53,6 +53,15 @@ def ordinal(k: int) -> str:
     suffix = "th" if 10 <= k % 100 <= 20 else {1: "st", 2: "nd", 3: "rd"}.get(k % 10, "th")
     return f"{k}{suffix}"
 
+def emit(line: dict, details: dict) -> None:
+    """The result line on standard output; the whole lines of the other workloads and comparisons,
+    which ``config.summary`` condenses, as one JSON object on standard error. With them the line had
+    grown to 20 KB, more than a reader of the end of the output keeps."""
+    if details:
+        print(json.dumps({"details": details}), file=sys.stderr, flush=True)
+    print(json.dumps(line), flush=True)
+
+
 def algorithmic_flops(stats: dict) -> float:
     return FLOP_PER_ATTEMPT * stats["attempts"] + FLOP_PER_ACCEPT * stats["accepted"] + FLOP_PER_RAY * stats["photons"]
 
@@ -648,6 +657,7 @@ def run_ours(args) -> None:
     peak64 = _lib.fma_peak_tflops(local, True)
 
     extra: dict = {}
+    details: dict = {}
     summary: dict = {}
     single = world == 1 and not args.kernel_only
     cpu = None
@@ -688,7 +698,7 @@ def run_ours(args) -> None:
                                                                 sweep.offsets)
         for name in ("spin99_1024", "spin99_2048"):
             m = mixed_vs_plain(K, local, stream, flush, name, oracle_check=not args.no_cpu)
-            extra[f"mixed_vs_plain_{name[-4:]}"] = m
+            details[f"mixed_vs_plain_{name[-4:]}"] = m
             summary[f"mixed_{name[-4:]}"] = {
                 "speedup_vs_plain_fp64": m["speedup_mixed_vs_plain"],
                 "near_band_speedup_vs_plain_fp64": m["speedup_mixed_near_vs_plain"],
@@ -736,14 +746,14 @@ def run_ours(args) -> None:
     if single and args.workload == "sweep":
         # The other two headline workloads, each with its own roofline and CPU baseline.
         bis = bisect_line(K, argparse.Namespace(steps=3, warmup=3, no_cpu=args.no_cpu, precision="fast64"))
-        extra["bisect"] = bis
+        details["bisect"] = bis
         summary["bisect"] = {"rays_s": bis["value"], "frac_fp64": bis["roofline"]["frac"],
                              "cpu_rays_s": (bis["cpu_baseline"] or {}).get("value"),
                              "edge_rms_over_rtol_median": {k: v["rms_over_rtol_median"]
                                                            for k, v in bis["edge_error_vs_bardeen"].items()}}
         torch.cuda.empty_cache()
         lens = lensing_line(K, argparse.Namespace(steps=3, warmup=3, no_cpu=args.no_cpu))
-        extra["lensing"] = lens
+        details["lensing"] = lens
         summary["lensing"] = {"rays_s": lens["value"], "e2e_rays_s": lens["e2e"]["value"],
                               "frac_fp64": (lens["roofline"] or {}).get("frac"),
                               "cpu_rays_s": (lens["cpu_baseline"] or {}).get("value"),
@@ -779,7 +789,7 @@ def run_ours(args) -> None:
                       "lane_occupancy": stats["busy_slots"] / max(stats["lane_slots"], 1)},
             **extra,
         }
-        print(json.dumps(line), flush=True)
+        emit(line, details)
     if world > 1:
         dist.destroy_process_group()
 
