@@ -2,24 +2,25 @@
 // and a few host threads.
 //
 // The driver copies pageable memory through a buffer of its own, one thread, one array after the
-// other, and the pages of a freshly allocated result are faulted in by that thread as well: 5-6 GB/s
-// where they are, 17 GB/s where the memory is reused, with a wait per array.  Here the transfers are
-// cut into pieces that go through a ring of pinned slots at the bus's rate (50 GB/s), while worker
-// threads move the pieces between the slots and the arrays (and take the page faults in parallel), and
-// one wait serves all arrays.  End to end, fast64 at rtol 1e-6, medians, with the driver's copies and
-// with these: 128^2 photons (2 MB of results) 1.10 and 0.86 ms, 256^2 (8 MB) 1.77 and 1.65, 300^2
-// 2.23 and 1.92, 400^2 3.48 and 2.87, 700^2 9.24 and 6.00, 1000^2 42.6 and 14.4.
-// Threads: one below 8 MB, two to 16 MB, one per 2 MB beyond, at most 12.  A thread per 2 MB from the
-// start made calls of 5 to 16 MB vary from call to call, by up to two (mixed precision, 256^2: 1.04 to
-// 1.95 ms, median 1.48-1.65; by this rule 1.30-1.37, by the driver 1.43-1.48), whether the workers were
-// new, waiting or joined; large transfers gain from all of them (92 MB of camera states at best 19.5 ms
-// by the driver, 3.8 by 12 threads, 5.3 by 6; a 1000^2 image 11.6 ms by 12, 13.1 by 6).
+// other, and the pages of a freshly allocated result are faulted in by that thread as well: 4-6 GB/s
+// into fresh pages, 17 GB/s into pages that a program gets back from its last result, and a wait per
+// array.  Here the transfers are cut into pieces that go through a ring of pinned slots at the bus's
+// rate (50 GB/s), while worker threads, one per 2 MB, move the pieces between the slots and the arrays
+// (and take the page faults in parallel), and one wait serves all arrays.  Medians end to end with the
+// driver's copies and with these, rtol 1e-6, results kept by the caller (fresh pages) and dropped:
+//   fast64  128^2 (2 MB)   1.95 -> 1.30 ms   1.09 -> 0.96     256^2 (8 MB)   4.70 -> 2.17   1.82 -> 1.75
+//           300^2 (11 MB)  6.20 -> 2.56      2.25 -> 1.99     400^2 (20 MB)  10.2 -> 3.55   3.5  -> 3.17
+//   2.9M photons with a pageable Y0 (189 MB in, 377 MB out) 126 -> 49 ms (trace 41).
+// Fewer threads below 16 MB (one per 8 MB) vary less from call to call and are up to a tenth faster into
+// reused pages, but up to half slower into fresh ones (256^2 2.85, 300^2 3.55 ms); six threads at most
+// instead of twelve take 13.1 ms instead of 11.6 for a 1000^2 image.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
@@ -54,7 +55,7 @@ class Staging {
  public:
   static constexpr size_t kSlotBytes = (size_t)1 << 20;
   static constexpr int kSlots = 32, kGroup = 4;
-  static constexpr size_t kFew = (size_t)1 << 24;  // a transfer below this takes one thread or two
+  static constexpr size_t kBytesPerThread = (size_t)1 << 21;  // a thread more per 2 MB, up to kThreads
   static constexpr int kThreads = 12;
 
   // Device to host arrays, after what `s` holds now; returns when every byte is in place.
@@ -143,8 +144,6 @@ class Staging {
     }
     const int n = (int)pieces.size();
     if (n == 0) return out ? cudaStreamSynchronize(s) : cudaSuccess;
-    // One array, and no values to check on the way: the driver's copy overlaps its own staging.
-    if (!bad && spans.size() == 1 && total < kFew) return copy_plain(spans, s, out, nullptr);
     ensure(n);
     if (have_ == 0) return copy_plain(spans, s, out, bad);
     const int slots = std::min(n, have_);
@@ -203,20 +202,23 @@ class Staging {
     if (out)
       for (int i = 0; i < slots && idle(i); ++i) queue_piece(i);
     const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-    const int threads = (int)std::min<size_t>((size_t)std::min(kThreads, hw),
-                                              total < kFew ? 1 + total / (kFew / 2) : total / (kFew / 8));
+    const int threads = (int)std::min<size_t>((size_t)std::min(kThreads, hw), 1 + total / kBytesPerThread);
     // The workers of an out() sleep until the first piece has arrived: a trace of any length may run
-    // ahead of the copies, and a thread that waits for an event keeps a core busy.
+    // ahead of the copies, and a thread that waits for an event keeps a core busy.  They watch for 0.2 ms
+    // first, since waking up takes that long (camera states of 400^2 0.36 ms, 0.62 by sleeping workers).
+    constexpr auto kWatch = std::chrono::microseconds(200);
     std::mutex gate;
     std::condition_variable opened;
-    bool open = !out;
+    std::atomic<bool> open{!out};
     std::vector<std::thread> pool;
     for (int t = 1; t < threads; ++t) {
       try {
         pool.emplace_back([&] {
+          const auto until = std::chrono::steady_clock::now() + kWatch;
+          while (!open.load() && std::chrono::steady_clock::now() < until) std::this_thread::yield();
           {
             std::unique_lock<std::mutex> lk(gate);
-            opened.wait(lk, [&] { return open; });
+            opened.wait(lk, [&] { return open.load(); });
           }
           cudaSetDevice(device);
           work();
@@ -229,7 +231,7 @@ class Staging {
       wait_slot(0);
       {
         std::lock_guard<std::mutex> lk(gate);
-        open = true;
+        open.store(true);
       }
       opened.notify_all();
     }

@@ -7,7 +7,6 @@ kernel running ahead of the copies): events then complete when it is let go.
 
 from __future__ import annotations
 
-import os
 import subprocess
 
 import pytest
@@ -32,7 +31,7 @@ struct FakeEvent { std::atomic<bool> recorded{false}; };
 using cudaEvent_t = FakeEvent*;
 constexpr unsigned cudaHostAllocDefault = 0, cudaEventDisableTiming = 2;
 namespace fake {
-inline std::atomic<int> allocs{1 << 30}, events{1 << 30}, made{0}, freed{0}, direct{0}, workers{0}, waiting{0}, most_waiting{0};
+inline std::atomic<int> allocs{1 << 30}, events{1 << 30}, made{0}, freed{0}, direct{0}, waiting{0}, most_waiting{0};
 inline std::atomic<bool> held{false};
 inline std::vector<char*> blocks;
 inline std::vector<double>* poisoned = nullptr;  // another thread's array: it turns to NaN when the first copy is queued
@@ -79,7 +78,7 @@ inline cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void
   return cudaSuccess;
 }
 inline cudaError_t cudaGetLastError() { return cudaSuccess; }
-inline cudaError_t cudaSetDevice(int) { return ++fake::workers, cudaSuccess; }
+inline cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 """
 
 PROGRAM = r"""
@@ -120,14 +119,6 @@ int main(int argc, char** argv) {
     bool finite = true;
     for (double x : b) finite = finite && std::isfinite(x);
     std::printf("ok %d sound %d\n", (int)ok, (int)(bad || finite));
-  } else if (argc > 3) {  // the workers and the driver's copies of a transfer of argv[2] arrays of argv[3] doubles
-    std::vector<std::vector<double>> a(std::atoi(argv[2]), std::vector<double>(std::atoll(argv[3]), 1.0)), b = a;
-    std::vector<krr_host::CopySpan> spans;
-    for (size_t k = 0; k < a.size(); ++k) spans.push_back({b[k].data(), a[k].data(), a[k].size() * 8});
-    std::atomic<bool> bad{false};
-    const bool checked = std::atoi(argv[1]) == 2;
-    const cudaError_t e = std::atoi(argv[1]) == 0 ? staging.out(0, spans, 0) : staging.in(0, spans, 0, checked ? &bad : nullptr);
-    std::printf("ok %d workers %d direct %d\n", (int)(e == cudaSuccess), (int)fake::workers, (int)fake::direct);
   } else if (argc > 2) {
     fake::allocs = std::atoi(argv[1]);
     fake::events = std::atoi(argv[2]);
@@ -182,25 +173,6 @@ def test_transfers_do_with_the_pinned_memory_there_is(program, allocs, events, d
 def test_one_thread_waits_for_the_trace(program):
     """A 32 MB result behind a kernel: twelve threads may copy, one may wait for the kernel's end."""
     assert _run(program) == ["waiting", "1", "ok", "1"]
-
-
-@pytest.mark.parametrize("way,arrays,doubles,workers,direct", [
-    (0, 9, 65536, 0, 0),        # 4.7 MB: the calling thread
-    (0, 9, 131072, 1, 0),       # 9.4 MB
-    (0, 9, 233016, 1, 0),       # just below 16 MB
-    (0, 9, 233017, 7, 0),
-    (0, 9, 1310720, 11, 0),     # 94 MB
-    (0, 1, 2097151, 0, 1),      # one array below 16 MB: the driver's copy
-    (0, 1, 2097152, 7, 0),
-    (1, 1, 2097151, 0, 1),
-    (2, 1, 1048575, 0, 0),      # its values are checked on the way
-    (2, 1, 2097151, 1, 0),
-    (1, 1, 16777216, 11, 0),
-])
-def test_threads_by_the_size_of_a_transfer(program, way, arrays, doubles, workers, direct):
-    """A thread more costs a short call more than it saves; workers that find no piece left count as well."""
-    most = min(12, os.cpu_count() or 1) - 1
-    assert _run(program, way, arrays, doubles) == ["ok", "1", "workers", str(min(workers, most)), "direct", str(direct)]
 
 
 @pytest.mark.parametrize("doubles", [1000, 131072])
